@@ -23,6 +23,7 @@
 // No kernel here traps: out-of-range ids set RS_DEV_OOB_ROW in the status word and are skipped.
 #include <cuda_bf16.h>
 #include <cstdlib>
+#include "common/row_vec.cuh"
 #include "common/rs_common.h"
 #include "comm/flags.cuh"
 #include "kv/hash_table.cuh"
@@ -86,9 +87,8 @@ __device__ __forceinline__ void store_pooled(const EmbFwdArgs& a, int t, int b, 
   }
 }
 
-// One warp per block of 32 consecutive bags of one table.  Lane i first resolves the metadata of
-// bag i (id range, and for single-id bags the row itself) with coalesced loads; the rows are then
-// fetched 8 bags at a time so that every warp keeps 8 independent 512-byte reads in flight.
+// Bags of a row-sharded table (fixed-capacity regions filled by the peers, compact occurrence list): one warp per block of
+// 32 consecutive bags of one table; lane i resolves the metadata of bag i.
 template <int NC>
 __device__ __forceinline__ void emb_fwd_body(const EmbFwdArgs& a, long long blk) {
   const int lane = threadIdx.x & 31;
@@ -128,35 +128,6 @@ __device__ __forceinline__ void emb_fwd_body(const EmbFwdArgs& a, long long blk)
     if (a.status) atomicOr(a.status, (unsigned long long)RS_DEV_OOB_ROW);
     return -1;
   };
-  const bool single = a.counts == nullptr && a.occ_cursor == nullptr && __all_sync(0xffffffffu, lane >= nb || end - beg == 1);
-  if (single && a.psw == nullptr) {
-    long long my_row = -1;
-    if (lane < nb) {
-      const long long id = a.indices[beg];
-      my_row = resolve(id);
-      if (a.row_idx) a.row_idx[beg] = my_row;
-      if (a.occ2bag) a.occ2bag[beg] = static_cast<int>(static_cast<long long>(t) * a.B + b0 + lane);
-    }
-    for (int j0 = 0; j0 < nb; j0 += 8) {
-      float4 x[8][NC];
-#pragma unroll
-      for (int u = 0; u < 8; ++u) {
-        const long long r = __shfl_sync(0xffffffffu, my_row, (j0 + u) & 31);
-#pragma unroll
-        for (int c = 0; c < NC; ++c) {
-          const int v = lane + c * 32;
-          x[u][c] = (j0 + u < nb && r >= 0 && v < nvec) ? __ldg(reinterpret_cast<const float4*>(a.weight + r * a.D) + v)
-                                                        : make_float4(0.f, 0.f, 0.f, 0.f);
-        }
-      }
-#pragma unroll
-      for (int u = 0; u < 8; ++u)
-        if (j0 + u < nb) store_pooled<NC>(a, t, b0 + j0 + u, x[u], lane, nvec);
-    }
-    return;
-  }
-
-  // General path: pooled bags (several ids, optional per-sample weights).
   for (int j = 0; j < nb; ++j) {
     const long long jb = __shfl_sync(0xffffffffu, beg, j);
     const long long je = __shfl_sync(0xffffffffu, end, j);
@@ -213,13 +184,230 @@ __device__ __forceinline__ void emb_fwd_body(const EmbFwdArgs& a, long long blk)
 }
 
 template <int NC>
-__global__ void __launch_bounds__(256) emb_fwd_kernel(const EmbFwdArgs a) {
+__global__ void __launch_bounds__(256) emb_fwd_sharded_kernel(const EmbFwdArgs a) {
   // Warps loop over the blocks of 32 bags, so the grid can be a single resident wave (see launch_emb_fwd).
   const int warps_per_block = blockDim.x >> 5;
   const long long total = static_cast<long long>(a.T) * ((a.B + 31) >> 5);
   const long long stride = static_cast<long long>(gridDim.x) * warps_per_block;
   for (long long blk = static_cast<long long>(blockIdx.x) * warps_per_block + (threadIdx.x >> 5); blk < total; blk += stride)
     emb_fwd_body<NC>(a, blk);
+  rs::flag_publish_when_grid_done(a.sig);   // (no-op without a signal) every thread arrives here
+}
+
+// Bags a sub-warp of L lanes takes at once: as many as its lanes can describe while their ids stay near one id per lane of a
+// warp, one bag from 17 ids on, never more than `cap`.
+template <int L> __device__ __forceinline__ int bags_per_task(long long h, int cap) {
+  int nb = h <= 1 ? L : (h >= 17 ? 1 : 1 << (31 - __clz(static_cast<int>(32 / h))));
+  nb = nb < L ? nb : L;
+  return nb < cap ? nb : cap;
+}
+
+// Lookup of whole tables.  A sub-warp of L lanes takes a task: up to L consecutive bags of one table, fewer where bags hold
+// several ids (see bags_per_task), so a table with 100 ids per bag spreads over as many sub-warps as it has bags.  Tasks are
+// numbered table after table; a warp finds the tables of its tasks in a running sum over the tables' task counts, 32 tables
+// per step.  Bags with one id each take the short way: all rows of a task in groups of U loads, straight to their places.
+// Otherwise the ids of the task's bags, which lie one after another, are walked in chunks of L with U rows in flight and a
+// bag is stored when its last id has been added.
+// Bound by issue slots and rows in flight (skewed ids hit L2): at 128 floats half a warp per row, 32-byte loads and 16-byte
+// bf16 stores.  The form before it (a warp per 32 bags whatever they held, 16-byte loads by a warp per row, destination
+// worked out per row) took 180 us for 65,536 x 26 one-id bags at Zipf 1.2 and 342 us for 8,192 x 26 bags of 214 ids a
+// sample, there with one table's 256 warps still running long after the others had ended.
+template <int V, int L, int NC>
+__global__ void __launch_bounds__(256, 3) emb_pool_kernel(const EmbFwdArgs a, const int nb_cap) {
+  constexpr int G = 32 / L;
+  constexpr int U = V * NC <= 8 ? 4 : 2;
+  constexpr unsigned kAll = 0xffffffffu;
+  const int lane = threadIdx.x & 31, l = lane & (L - 1), g = lane / L;
+  const unsigned wm = L == 32 ? kAll : ((1u << (L & 31)) - 1u) << (g * L);
+  const unsigned stride = gridDim.x * (blockDim.x >> 5) * G;
+  const int nvec = a.D / V;
+  const int esz = a.out_bf16 ? 2 : 4;
+
+  int jag_nb = 0;
+  if (a.offsets) {
+    const long long bags = static_cast<long long>(a.T) * a.B;
+    jag_nb = bags_per_task<L>((a.offsets[bags] - a.offsets[0] + bags - 1) / bags, nb_cap);
+  }
+  // Lane i: bags per task and running task count of table tab0 + i.
+  int tab0 = 0, my_nb = 1;
+  unsigned my_end = 0;
+  auto load_tables = [&](int first, unsigned before) {
+    tab0 = first;
+    const int t = first + lane;
+    my_nb = 1;
+    unsigned n = 0;
+    if (t < a.T) {
+      my_nb = a.offsets ? jag_nb : bags_per_task<L>(a.hotness[t], nb_cap);
+      n = static_cast<unsigned>((a.B + my_nb - 1) / my_nb);
+    }
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const unsigned y = __shfl_up_sync(kAll, n, o);
+      if (lane >= o) n += y;
+    }
+    my_end = before + n;
+  };
+  load_tables(0, 0);
+  unsigned before = 0;                                   // tasks of the tables below tab0
+
+  for (unsigned base = (blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5)) * G;; base += stride) {
+    const unsigned task = base + g;
+    // Tables of the warp's tasks.  They ascend, so a step to the next 32 tables is never taken back; a warp whose tasks lie
+    // on both sides of such a step serves the lower ones first.
+    bool todo = true;
+    bool more = true;
+    while (more) {
+      const unsigned last = __shfl_sync(kAll, my_end, 31);
+      const bool here = todo && task < last;
+      int pos = 0;
+#pragma unroll
+      for (int st = 16; st > 0; st >>= 1) {
+        const unsigned c = __shfl_sync(kAll, my_end, pos + st - 1);
+        if (c <= task) pos += st;
+      }
+      const unsigned prev = __shfl_sync(kAll, my_end, pos > 0 ? pos - 1 : 0);
+      const int nb = __shfl_sync(kAll, my_nb, pos);
+      if (here) {
+        todo = false;
+        const int t = tab0 + pos;
+        const int b0 = static_cast<int>((task - (pos > 0 ? prev : before)) * static_cast<unsigned>(nb));
+        const int n = min(nb, a.B - b0);
+        const long long tbase = a.table_base[t], nrows = a.table_rows[t];
+        long long beg = 0, end = 0;
+        if (l < n) {
+          if (a.offsets) {
+            const long long bag = static_cast<long long>(t) * a.B + b0 + l;
+            beg = a.offsets[bag];
+            end = a.offsets[bag + 1];
+          } else {
+            const int h = a.hotness[t];
+            beg = a.hot_base[t] + static_cast<long long>(b0 + l) * h;
+            end = beg + h;
+          }
+        }
+        auto resolve = [&](long long id) -> long long {
+          if (a.use_hash) return rs::ht_find(a.ht, static_cast<unsigned long long>(id));
+          if (id >= 0 && id < nrows) return tbase + id;
+          if (a.status) atomicOr(a.status, (unsigned long long)RS_DEV_OOB_ROW);
+          return -1;
+        };
+        // Where the bags go: all to one rank (one base for the task) unless the task straddles two ranks' samples.
+        const int col = a.dst_col[t];
+        const int rank0 = b0 / a.B_local;
+        const bool one_rank = (b0 + n - 1) < (rank0 + 1) * static_cast<long long>(a.B_local);
+        char* const dst0 = reinterpret_cast<char*>(a.dst[rank0]) +
+                           ((b0 - rank0 * static_cast<long long>(a.B_local)) * a.dst_row_stride + col) * esz;
+        auto place = [&](int j) -> char* {
+          if (one_rank) return dst0 + j * (a.dst_row_stride * esz);
+          const int r = (b0 + j) / a.B_local;
+          return reinterpret_cast<char*>(a.dst[r]) + ((b0 + j - r * static_cast<long long>(a.B_local)) * a.dst_row_stride + col) * esz;
+        };
+        auto store = [&](int j, const rs::RowVec<V> (&x)[NC]) {
+          char* const d = place(j);
+          const bool al = (reinterpret_cast<uintptr_t>(d) & 15) == 0;
+#pragma unroll
+          for (int c = 0; c < NC; ++c) {
+            const int v = l + c * L;
+            if (v < nvec) {
+              if (a.out_bf16) rs::row_store_bf16(reinterpret_cast<__nv_bfloat16*>(d) + v * V, x[c], al);
+              else rs::row_store(reinterpret_cast<float*>(d) + v * V, x[c]);
+            }
+          }
+        };
+        const int bag0 = t * a.B + b0;                    // (T * B < 2^31, checked on the host)
+        if (a.psw == nullptr && __all_sync(wm, l >= n || end - beg == 1)) {
+          long long my_row = -1;
+          if (l < n) {
+            my_row = resolve(a.indices[beg]);
+            if (a.row_idx) a.row_idx[beg] = my_row;
+            if (a.occ2bag) a.occ2bag[beg] = bag0 + l;
+          }
+          for (int j0 = 0; j0 < n; j0 += U) {
+            rs::RowVec<V> x[U][NC];
+#pragma unroll
+            for (int u = 0; u < U; ++u) {
+              const long long r = __shfl_sync(wm, my_row, (j0 + u) & (L - 1), L);
+#pragma unroll
+              for (int c = 0; c < NC; ++c) {
+                rs::row_zero(x[u][c]);
+                const int v = l + c * L;
+                if (j0 + u < n && r >= 0 && v < nvec) rs::row_load_nc(x[u][c], a.weight + r * a.D + v * V);
+              }
+            }
+#pragma unroll
+            for (int u = 0; u < U; ++u)
+              if (j0 + u < n) store(j0 + u, x[u]);
+          }
+        } else {
+          rs::RowVec<V> acc[NC];
+#pragma unroll
+          for (int c = 0; c < NC; ++c) rs::row_zero(acc[c]);
+          const long long i_begin = __shfl_sync(wm, beg, 0, L), i_end = __shfl_sync(wm, end, n - 1, L);
+          int j = 0;                                      // bag being summed and the end of its ids
+          long long j_end = __shfl_sync(wm, end, 0, L);
+          auto close = [&]() {
+            store(j, acc);
+#pragma unroll
+            for (int c = 0; c < NC; ++c) rs::row_zero(acc[c]);
+            ++j;
+            j_end = __shfl_sync(wm, end, j & (L - 1), L);
+          };
+          for (long long i0 = i_begin; i0 < i_end; i0 += L) {
+            const int m = static_cast<int>(min(static_cast<long long>(L), i_end - i0));
+            long long my_row = -1;
+            float my_w = 1.f;
+            // lane l's id belongs to the first bag that ends behind it
+            int mine = 0;
+#pragma unroll
+            for (int st = L / 2; st > 0; st >>= 1) {
+              const long long e = __shfl_sync(wm, end, min(mine + st, n) - 1, L);
+              if (mine + st <= n - 1 && e <= i0 + l) mine += st;
+            }
+            if (l < m) {
+              my_row = resolve(a.indices[i0 + l]);
+              if (a.psw) my_w = a.psw[i0 + l];
+              if (a.row_idx) a.row_idx[i0 + l] = my_row;
+              if (a.occ2bag) a.occ2bag[i0 + l] = bag0 + mine;
+            }
+            for (int k0 = 0; k0 < m; k0 += U) {
+              rs::RowVec<V> x[U][NC];
+              float w[U];
+#pragma unroll
+              for (int u = 0; u < U; ++u) {
+                const long long r = __shfl_sync(wm, my_row, (k0 + u) & (L - 1), L);
+                w[u] = __shfl_sync(wm, my_w, (k0 + u) & (L - 1), L);
+#pragma unroll
+                for (int c = 0; c < NC; ++c) {
+                  rs::row_zero(x[u][c]);
+                  const int v = l + c * L;
+                  if (k0 + u < m && r >= 0 && v < nvec) rs::row_load_nc(x[u][c], a.weight + r * a.D + v * V);
+                }
+              }
+#pragma unroll
+              for (int u = 0; u < U; ++u) {
+                if (k0 + u >= m) break;
+                while (j < n - 1 && i0 + k0 + u >= j_end) close();
+#pragma unroll
+                for (int c = 0; c < NC; ++c)
+#pragma unroll
+                  for (int e = 0; e < V; ++e) acc[c].v[e] = fmaf(w[u], x[u][c].v[e], acc[c].v[e]);
+              }
+            }
+          }
+          while (j < n) close();                          // the last bag with ids, and the empty ones after it
+        }
+      }
+      __syncwarp();
+      // Another 32 tables when a task of this warp lies behind these.
+      more = __any_sync(kAll, todo && task >= last) && tab0 + 32 < a.T;
+      if (more) {
+        before = last;
+        load_tables(tab0 + 32, before);
+      }
+    }
+    // The last table's count is known once it is loaded: a warp none of whose tasks exist is done.
+    if (!__any_sync(kAll, !todo)) break;
+  }
   rs::flag_publish_when_grid_done(a.sig);   // (no-op without a signal) every thread arrives here
 }
 
@@ -251,166 +439,171 @@ __device__ __forceinline__ long long live_nnz(const EmbBwdArgs& a) {
   return n < a.nnz ? n : a.nnz;
 }
 
-constexpr int kGroup = 256;
-constexpr int kSlots = 512;
+constexpr int kGroup = 256;      // threads of an apply CTA, and the most occurrences it takes
+constexpr int kSlots = 2 * kGroup;
 
-template <int NC>
-__device__ __forceinline__ void load_grad(const EmbBwdArgs& a, long long goff, int lane, int nvec, float4 (&g)[NC]) {
-#pragma unroll
-  for (int c = 0; c < NC; ++c) {
-    const int v = lane + c * 32;
-    if (v < nvec) {
-      if (a.grad_bf16) {
-        const uint2 raw = __ldg(reinterpret_cast<const uint2*>(reinterpret_cast<const __nv_bfloat16*>(a.grad) + goff) + v);
-        const float2 flo = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&raw.x));
-        const float2 fhi = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&raw.y));
-        g[c] = make_float4(flo.x, flo.y, fhi.x, fhi.y);
-      } else {
-        g[c] = __ldg(reinterpret_cast<const float4*>(reinterpret_cast<const float*>(a.grad) + goff) + v);
-      }
-    } else {
-      g[c] = make_float4(0.f, 0.f, 0.f, 0.f);
-    }
+// Sample and table of occurrence i.  32-bit arithmetic wherever the bag number allows it: a 64-bit division costs more
+// than the rest of the address computation.
+__device__ __forceinline__ void bag_of(const EmbBwdArgs& a, long long i, int& t, int& b) {
+  if (a.occ2bag) {
+    const unsigned bag = static_cast<unsigned>(a.occ2bag[i]);
+    t = static_cast<int>(bag / static_cast<unsigned>(a.B));
+    b = static_cast<int>(bag - static_cast<unsigned>(t) * static_cast<unsigned>(a.B));
+  } else if (i < a.B) {
+    t = 0;
+    b = static_cast<int>(i);
+  } else {
+    t = static_cast<int>(i / a.B);
+    b = static_cast<int>(i % a.B);
   }
 }
 
 // Pass 1 of row-wise Adagrad: state[row] += w^2 * |g_bag|^2 / D for every occurrence.
-// With precomputed bag norms this is one thread per occurrence; otherwise one warp per occurrence.
-template <int NC>
-__global__ void __launch_bounds__(256) emb_state_kernel(const EmbBwdArgs a) {
-  const float inv_d = 1.f / static_cast<float>(a.D);
+// With precomputed bag norms it is one thread per occurrence; the lanes of a warp that hold the same row add up in
+// registers first, so a warp sends one atomic per distinct row.  Bound by the issue of the chain steps and by the scattered
+// 4-byte norms.  It replaced a shared-memory hash whose float adds are compare-and-swap loops that the hot rows of a skewed
+// id stream serialise: 1.70 M occurrences at Zipf 1.2 took 49 us.
+__global__ void __launch_bounds__(256) emb_state_norm_kernel(const EmbBwdArgs a) {
   const long long nnz = live_nnz(a);
-  if (a.gnorm) {
-    if (static_cast<long long>(blockIdx.x) * blockDim.x >= nnz) return;   // whole block past the live occurrences
-    rs::flag_wait_all(a.wait);
-    // One thread per occurrence; equal rows of the block are combined in a shared-memory hash first, so a hot
-    // row costs one global atomic per block instead of one per occurrence.
-    __shared__ long long s_key[kSlots];
-    __shared__ float s_val[kSlots];
-    for (int s = threadIdx.x; s < kSlots; s += blockDim.x) {
-      s_key[s] = -1;
-      s_val[s] = 0.f;
-    }
-    __syncthreads();
-    const long long i = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x;
-    if (i < nnz) {
-      const long long row = a.row_idx[i];
-      if (row >= 0 && row < a.total_rows) {
-        const long long bag = a.occ2bag ? a.occ2bag[i] : i;
-        const int t = static_cast<int>(bag / a.B);
-        const long long b = bag % a.B;
-        const float w = a.psw ? a.psw[i] : 1.f;
-        const float v = w * w * a.gnorm[b * a.gnorm_stride + t] * inv_d;
-        unsigned s = static_cast<unsigned>(rs::ht_hash(static_cast<unsigned long long>(row))) & (kSlots - 1);
-        for (int p = 0; p < kSlots; ++p) {
-          const long long prev = static_cast<long long>(atomicCAS(reinterpret_cast<unsigned long long*>(&s_key[s]),
-                                                                   static_cast<unsigned long long>(-1ll),
-                                                                   static_cast<unsigned long long>(row)));
-          if (prev == -1 || prev == row) {
-            atomicAdd(&s_val[s], v);
-            break;
-          }
-          s = (s + 1) & (kSlots - 1);
-        }
-      }
-    }
-    __syncthreads();
-    for (int s = threadIdx.x; s < kSlots; s += blockDim.x)
-      if (s_key[s] >= 0) atomicAdd(&a.state[s_key[s]], s_val[s]);
-    return;
-  }
-  if (static_cast<long long>(blockIdx.x) * (blockDim.x >> 5) >= nnz) return;
+  if (static_cast<long long>(blockIdx.x) * blockDim.x >= nnz) return;   // whole block past the live occurrences
   rs::flag_wait_all(a.wait);
-  const long long i = static_cast<long long>(blockIdx.x) * (blockDim.x >> 5) + (threadIdx.x >> 5);
-  if (i >= nnz) return;
-  const int lane = threadIdx.x & 31;
-  const long long row = a.row_idx[i];
-  if (row < 0 || row >= a.total_rows) return;
-  const long long bag = a.occ2bag ? a.occ2bag[i] : i;
-  const int t = static_cast<int>(bag / a.B);
-  const long long b = bag % a.B;
-  const long long goff = b * a.grad_row_stride + (a.grad_col ? a.grad_col[t] : 0);
-  const float w = a.psw ? a.psw[i] : 1.f;
-  float4 g[NC];
-  load_grad<NC>(a, goff, lane, a.D >> 2, g);
-  float sq = 0.f;
-#pragma unroll
-  for (int c = 0; c < NC; ++c) sq += g[c].x * g[c].x + g[c].y * g[c].y + g[c].z * g[c].z + g[c].w * g[c].w;
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) sq += __shfl_xor_sync(0xffffffffu, sq, o);
-  if (lane == 0) atomicAdd(&a.state[row], w * w * sq * inv_d);
+  const float inv_d = 1.f / static_cast<float>(a.D);
+  const long long i = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x;
+  long long row = -1;
+  float v = 0.f;
+  if (i < nnz) {
+    row = a.row_idx[i];
+    if (row < 0 || row >= a.total_rows) {
+      row = -1;
+    } else {
+      int t, b;
+      bag_of(a, i, t, b);
+      const float w = a.psw ? a.psw[i] : 1.f;
+      v = w * w * a.gnorm[static_cast<long long>(b) * a.gnorm_stride + t] * inv_d;
+    }
+  }
+  const bool first = rs::warp_sum_equal_keys(static_cast<unsigned long long>(row), v);
+  if (first && row >= 0) atomicAdd(&a.state[row], v);
 }
 
-// Apply pass: one CTA per group of 256 occurrences.  The group is counting-sorted by row in shared memory (hash
-// slot -> count -> exclusive scan -> position), so equal rows sit next to each other.  Every warp then owns 32
-// consecutive sorted positions, whatever the skew of the ids: it streams their gradients with kApplyInFlight
-// loads (and the matching Adagrad states) in flight, sums runs of equal rows in registers and issues one vector
-// atomic per run.  A row that straddles warps or groups simply receives several atomics.
-constexpr int kApplyInFlight = 8;
+// Without norms a warp takes `opw` consecutive occurrences (32, or 8 when the batch would leave SMs without work): its
+// sub-warps compute the squared norms, U gradient rows of each in flight, and the lanes then add up as above.
+template <int V, int L, int NC, bool BF16>
+__global__ void __launch_bounds__(256) emb_state_kernel(const EmbBwdArgs a, const int opw) {
+  constexpr int G = 32 / L;
+  constexpr int U = V * NC <= 8 ? 4 : 2;
+  const long long nnz = live_nnz(a);
+  const long long i0 = (static_cast<long long>(blockIdx.x) * (blockDim.x >> 5) + (threadIdx.x >> 5)) * opw;
+  if (static_cast<long long>(blockIdx.x) * (blockDim.x >> 5) * opw >= nnz) return;
+  rs::flag_wait_all(a.wait);
+  const int lane = threadIdx.x & 31, l = lane & (L - 1), g = lane / L;
+  const long long i = i0 + lane;
+  long long row = -1, goff = 0;
+  float w = 1.f, v = 0.f;
+  if (lane < opw && i < nnz) {
+    row = a.row_idx[i];
+    if (row >= a.total_rows) row = -1;
+    if (row >= 0) {
+      int t, b;
+      bag_of(a, i, t, b);
+      goff = b * a.grad_row_stride + (a.grad_col ? a.grad_col[t] : 0);
+      if (a.psw) w = a.psw[i];
+    } else {
+      row = -1;
+    }
+  }
+  const bool wide = V == 4 || __all_sync(0xffffffffu, (goff & 7) == 0);
+  const int nvec = a.D / V;
+  for (int j0 = 0; j0 < opw; j0 += G * U) {
+    rs::RawVec<V, BF16> x[U][NC];
+    bool on[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const int j = (j0 + u * G + g) & 31;
+      const long long go = __shfl_sync(0xffffffffu, goff, j);
+      on[u] = __shfl_sync(0xffffffffu, row, j) >= 0 && j0 + u * G + g < opw;
+      if (on[u]) {
+#pragma unroll
+        for (int c = 0; c < NC; ++c) x[u][c].load(a.grad, go + static_cast<long long>(min(l + c * L, nvec - 1)) * V, wide);
+      }
+    }
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      float sq = 0.f;
+      if (on[u]) {
+#pragma unroll
+        for (int c = 0; c < NC; ++c) {
+          if (l + c * L < nvec) {
+            const rs::RowVec<V> f = x[u][c].get();
+#pragma unroll
+            for (int e = 0; e < V; ++e) sq += f.v[e] * f.v[e];
+          }
+        }
+      }
+#pragma unroll
+      for (int o = L / 2; o > 0; o >>= 1) sq += __shfl_xor_sync(0xffffffffu, sq, o);
+      // occurrence j0 + u * G + k lies in sub-warp k; lane j keeps the norm of occurrence j
+      const int k = lane - j0 - u * G;
+      const float got = __shfl_sync(0xffffffffu, sq, (k & (G - 1)) * L);
+      if (k >= 0 && k < G) v = got;
+    }
+  }
+  v *= w * w / static_cast<float>(a.D);
+  const bool first = rs::warp_sum_equal_keys(static_cast<unsigned long long>(row), v);
+  if (first && row >= 0) atomicAdd(&a.state[row], v);
+}
 
-// Raw (unconverted) gradient chunk: the loads of a batch are issued back to back with no branch and no use of
-// their results in between, so all of them are in flight together; conversion happens when they are consumed.
-template <bool BF16> struct RawGrad;
-template <> struct RawGrad<true> {
-  uint2 v;
-  __device__ __forceinline__ void load(const void* base, long long goff, int vec) {
-    v = __ldg(reinterpret_cast<const uint2*>(reinterpret_cast<const __nv_bfloat16*>(base) + goff) + vec);
-  }
-  __device__ __forceinline__ float4 get() const {
-    const float2 lo = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&v.x));
-    const float2 hi = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&v.y));
-    return make_float4(lo.x, lo.y, hi.x, hi.y);
-  }
-};
-template <> struct RawGrad<false> {
-  float4 v;
-  __device__ __forceinline__ void load(const void* base, long long goff, int vec) {
-    v = __ldg(reinterpret_cast<const float4*>(reinterpret_cast<const float*>(base) + goff) + vec);
-  }
-  __device__ __forceinline__ float4 get() const { return v; }
-};
-
-template <int NC, bool BF16>
-__global__ void __launch_bounds__(kGroup) emb_apply_kernel(const EmbBwdArgs a) {
+// Apply pass: one CTA per `gs` occurrences (256, or 64 when that leaves SMs without work).  They are counting-sorted by row
+// in shared memory (hash slot -> count -> exclusive scan -> position), so equal rows sit next to each other, together with
+// their factor -lr * w / (sqrt(state) + eps): one state read and one root per occurrence, by the thread that owns it, and
+// none in the loop over the rows.  Every sub-warp then owns an equal share of the sorted positions, whatever the skew of the
+// ids: it streams their gradients with U loads in flight, sums runs of equal rows in registers and issues one vector
+// atomic per unit and run.  A row that straddles sub-warps or groups simply receives several atomics.
+// Bound by issue slots and latency: 16-byte bf16 loads by half a warp per 128-float row, at four or five CTAs per SM.  The
+// form before it (a warp per row, state read and root inside the loop, 76 registers, 32 % of the warps resident) took
+// 278 us for 1.70 M occurrences x 128 at Zipf 1.2.
+template <int V, int L, int NC, bool BF16>
+__global__ void __launch_bounds__(kGroup) emb_apply_kernel(const EmbBwdArgs a, const int gs) {
   __shared__ long long s_key[kSlots];
-  __shared__ int s_cnt[kSlots];        // occurrences per slot, then exclusive offsets
+  __shared__ int s_cnt[kSlots];         // occurrences per slot, then exclusive offsets
   __shared__ long long s_goff[kGroup];  // sorted: gradient offset
   __shared__ long long s_row[kGroup];   // sorted: row
-  __shared__ float s_w[kGroup];         // sorted: per-sample weight
+  __shared__ float s_coef[kGroup];      // sorted: factor of the gradient
   __shared__ int s_warp_sum[kGroup / 32];
-  __shared__ int s_total;
 
   const int tid = threadIdx.x;
   const int warp = tid >> 5, lane = tid & 31;
-  const long long g0 = static_cast<long long>(blockIdx.x) * kGroup;
+  const long long g0 = static_cast<long long>(blockIdx.x) * gs;
   const long long nnz = live_nnz(a);
   if (g0 >= nnz) return;                       // whole group past the live occurrences
   rs::flag_wait_all(a.wait);
-  for (int s = tid; s < kSlots; s += kGroup) {
+  const int slots = 2 * gs;
+  for (int s = tid; s < slots; s += kGroup) {
     s_key[s] = -1;
     s_cnt[s] = 0;
   }
-  __syncthreads();
-
   long long row = -1, goff = 0;
-  float w = 1.f;
+  float coef = -a.lr;
   int slot = -1, rank = 0;
-  if (g0 + tid < nnz) {
+  if (tid < gs && g0 + tid < nnz) {
     const long long occ = g0 + tid;
     row = a.row_idx[occ];
     if (row >= a.total_rows) {
       if (a.status) atomicOr(a.status, (unsigned long long)RS_DEV_OOB_ROW);
       row = -1;
     }
-    const long long bag = a.occ2bag ? a.occ2bag[occ] : occ;
-    const int t = static_cast<int>(bag / a.B);
-    const long long b = bag % a.B;
-    goff = b * a.grad_row_stride + (a.grad_col ? a.grad_col[t] : 0);
-    if (a.psw) w = a.psw[occ];
+    if (row >= 0) {
+      int t, b;
+      bag_of(a, occ, t, b);
+      goff = b * a.grad_row_stride + (a.grad_col ? a.grad_col[t] : 0);
+      if (a.optimizer == 1) coef = -a.lr / (sqrtf(__ldcv(&a.state[row])) + a.eps);
+      if (a.psw) coef *= a.psw[occ];
+    }
   }
+  const bool wide = !__syncthreads_or(V == 8 && (goff & 7) != 0);   // (also: the slots are cleared)
   if (row >= 0) {
-    unsigned s = static_cast<unsigned>(rs::ht_hash(static_cast<unsigned long long>(row))) & (kSlots - 1);
-    for (int p = 0; p < kSlots; ++p) {
+    unsigned s = static_cast<unsigned>(rs::ht_hash(static_cast<unsigned long long>(row))) & (slots - 1);
+    for (int p = 0; p < slots; ++p) {
       const long long prev = static_cast<long long>(atomicCAS(reinterpret_cast<unsigned long long*>(&s_key[s]),
                                                                static_cast<unsigned long long>(-1ll),
                                                                static_cast<unsigned long long>(row)));
@@ -419,13 +612,14 @@ __global__ void __launch_bounds__(kGroup) emb_apply_kernel(const EmbBwdArgs a) {
         rank = atomicAdd(&s_cnt[s], 1);
         break;
       }
-      s = (s + 1) & (kSlots - 1);
+      s = (s + 1) & (slots - 1);
     }
   }
   __syncthreads();
-  // exclusive scan of the 512 slot counts: two slots per thread, warp shuffles, then the warp totals
+  // exclusive scan of the slot counts: two slots per thread, warp shuffles, then the warp totals
   {
-    const int c0 = s_cnt[2 * tid], c1 = s_cnt[2 * tid + 1];
+    const bool mine = 2 * tid < slots;
+    const int c0 = mine ? s_cnt[2 * tid] : 0, c1 = mine ? s_cnt[2 * tid + 1] : 0;
     int incl = c0 + c1;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
@@ -438,73 +632,88 @@ __global__ void __launch_bounds__(kGroup) emb_apply_kernel(const EmbBwdArgs a) {
 #pragma unroll
     for (int q = 0; q < kGroup / 32; ++q) base += q < warp ? s_warp_sum[q] : 0;
     const int excl = base + incl - (c0 + c1);
-    s_cnt[2 * tid] = excl;
-    s_cnt[2 * tid + 1] = excl + c0;
-    if (tid == kGroup - 1) s_total = base + incl;
+    if (mine) {
+      s_cnt[2 * tid] = excl;
+      s_cnt[2 * tid + 1] = excl + c0;
+    }
   }
   __syncthreads();
   if (slot >= 0) {
     const int pos = s_cnt[slot] + rank;
     s_goff[pos] = goff;
     s_row[pos] = row;
-    s_w[pos] = w;
+    s_coef[pos] = coef;
   }
   __syncthreads();
 
-  const int total = s_total;
-  const int nvec = a.D >> 2;
-  const int p_end = min(total, warp * 32 + 32);
-  long long cur = -1;
-  float cur_state = 0.f;
-  float4 acc[NC];
+  constexpr int G = 32 / L;
+  constexpr int U = V * NC <= 8 ? 4 : 2;
+  int total = 0;
 #pragma unroll
-  for (int c = 0; c < NC; ++c) acc[c] = make_float4(0.f, 0.f, 0.f, 0.f);
+  for (int q = 0; q < kGroup / 32; ++q) total += s_warp_sum[q];
+  const int l = lane & (L - 1);
+  const int nvec = a.D / V;
+  const int share = gs / ((kGroup / 32) * G);
+  const int p_begin = (warp * G + lane / L) * share;
+  const int p_end = min(total, p_begin + share);
+  long long cur = -1;
+  rs::RowVec<V> acc[NC];
+#pragma unroll
+  for (int c = 0; c < NC; ++c) rs::row_zero(acc[c]);
 
   auto flush = [&]() {
     if (cur < 0) return;
-    float scale = -a.lr;
-    if (a.optimizer == 1) scale = -a.lr / (sqrtf(cur_state) + a.eps);
 #pragma unroll
     for (int c = 0; c < NC; ++c) {
-      const int v = lane + c * 32;
-      if (v < nvec) {
-        float4 u = make_float4(scale * acc[c].x, scale * acc[c].y, scale * acc[c].z, scale * acc[c].w);
-        atomicAdd(reinterpret_cast<float4*>(a.weight + cur * a.D) + v, u);
-      }
-      acc[c] = make_float4(0.f, 0.f, 0.f, 0.f);
+      const int v = l + c * L;
+      if (v < nvec) rs::row_atomic_add(a.weight + cur * a.D + static_cast<long long>(v) * V, acc[c]);
+      rs::row_zero(acc[c]);
     }
   };
 
-  constexpr int U = NC == 1 ? kApplyInFlight : (NC == 2 ? 4 : 2);
-  for (int p0 = warp * 32; p0 < p_end; p0 += U) {
-    RawGrad<BF16> g[U][NC];
-    float st[U];
-    long long r[U];
+  for (int p0 = p_begin; p0 < p_end; p0 += U) {
+    rs::RawVec<V, BF16> x[U][NC];
 #pragma unroll
     for (int u = 0; u < U; ++u) {
-      const int p = min(p0 + u, p_end - 1);   // past the end: re-read the last valid position, ignored below
-      r[u] = s_row[p];
-      const long long go = s_goff[p];
+      const long long go = s_goff[min(p0 + u, p_end - 1)];   // past the end: re-read the last valid position, ignored below
 #pragma unroll
-      for (int c = 0; c < NC; ++c) g[u][c].load(a.grad, go, min(lane + c * 32, nvec - 1));
-      st[u] = a.optimizer == 1 ? __ldcv(&a.state[r[u]]) : 0.f;
+      for (int c = 0; c < NC; ++c) x[u][c].load(a.grad, go + static_cast<long long>(min(l + c * L, nvec - 1)) * V, wide);
     }
 #pragma unroll
     for (int u = 0; u < U; ++u) {
       if (p0 + u >= p_end) break;
-      if (r[u] != cur) {
+      const long long r = s_row[p0 + u];
+      if (r != cur) {
         flush();
-        cur = r[u];
-        cur_state = st[u];
+        cur = r;
       }
-      const float wu = s_w[p0 + u];
+      const float k = s_coef[p0 + u];
 #pragma unroll
       for (int c = 0; c < NC; ++c) {
-        const float4 x = g[u][c].get();
-        acc[c].x += wu * x.x; acc[c].y += wu * x.y;
-        acc[c].z += wu * x.z; acc[c].w += wu * x.w;
+        const rs::RowVec<V> f = x[u][c].get();
+#pragma unroll
+        for (int e = 0; e < V; ++e) acc[c].v[e] = fmaf(k, f.v[e], acc[c].v[e]);
       }
     }
+  }
+  if (G > 1) {
+    // A hot row fills whole sub-warps: equal rows at the ends of neighbouring sub-warps are added up towards the first of
+    // them, which alone sends (a 32-float row has eight sub-warps of four positions each, and as many atomics otherwise).
+    __syncwarp();
+#pragma unroll
+    for (int o = 1; o < G; o <<= 1) {
+      const long long theirs = __shfl_down_sync(0xffffffffu, cur, o * L);
+      const bool join = lane + o * L < 32 && cur >= 0 && theirs == cur;
+#pragma unroll
+      for (int c = 0; c < NC; ++c)
+#pragma unroll
+        for (int e = 0; e < V; ++e) {
+          const float x = __shfl_down_sync(0xffffffffu, acc[c].v[e], o * L);
+          if (join) acc[c].v[e] += x;
+        }
+    }
+    const long long before = __shfl_up_sync(0xffffffffu, cur, L);
+    if (lane >= L && before == cur) cur = -1;
   }
   flush();
 }
@@ -553,21 +762,41 @@ __global__ void rows_scatter_kernel(float* __restrict__ w, const long long* __re
 namespace {
 int launch_emb_fwd(const EmbFwdArgs& a, cudaStream_t stream) {
   if (a.T == 0 || a.B == 0) return RS_OK;
-  const long long nblocks = static_cast<long long>(a.T) * ((a.B + 31) / 32);
   // Four warps per CTA: at 64 registers per thread such a CTA still fits on an SM beside one persistent GEMM CTA, so the
   // lookup and its NVLink pushes really run at the same time as the MLP that is launched beside them.
   static const int wpb = [] { const char* e = getenv("RECSTORE_EMB_FWD_WARPS"); return (e && e[0] == '8') ? 8 : 4; }();
-  long long grid = (nblocks + wpb - 1) / wpb;
-  // RECSTORE_EMB_FWD_CTAS_PER_SM=c (0 = one CTA per 4 or 8 blocks of bags, the default): at most c CTAs per SM, the
-  // warps looping over the bags.  The hardware hands out the CTAs of a later kernel only once every CTA of the earlier
-  // one has been placed, so a lookup with thousands of CTAs holds back the GEMMs launched beside it on another stream
-  // until its last wave; a grid that is resident as a whole does not.
+  // RECSTORE_EMB_FWD_CTAS_PER_SM=c (0 = no limit, the default): at most c CTAs per SM, the warps looping over the bags.
+  // The hardware hands out the CTAs of a later kernel only once every CTA of the earlier one has been placed, so a lookup
+  // with thousands of CTAs holds back the GEMMs launched beside it on another stream until its last wave; a grid that is
+  // resident as a whole does not.
   static const int per_sm = [] { const char* e = getenv("RECSTORE_EMB_FWD_CTAS_PER_SM"); return e ? atoi(e) : 0; }();
-  if (per_sm > 0 && grid > 148ll * per_sm) grid = 148ll * per_sm;
-  RS_REQUIRE(grid < (1ll << 31), "rs_emb_forward: too many bags");
-  if (a.D <= 128) emb_fwd_kernel<1><<<static_cast<unsigned>(grid), wpb * 32, 0, stream>>>(a);
-  else if (a.D <= 256) emb_fwd_kernel<2><<<static_cast<unsigned>(grid), wpb * 32, 0, stream>>>(a);
-  else emb_fwd_kernel<4><<<static_cast<unsigned>(grid), wpb * 32, 0, stream>>>(a);
+  const long long bags = static_cast<long long>(a.T) * a.B;
+  if (a.counts || a.occ_cursor || a.id_div > 1 || a.wait.my_flags || bags >= (1ll << 31)) {
+    const long long nblocks = static_cast<long long>(a.T) * ((a.B + 31) / 32);
+    long long grid = (nblocks + wpb - 1) / wpb;
+    if (per_sm > 0 && grid > 148ll * per_sm) grid = 148ll * per_sm;
+    RS_REQUIRE(grid < (1ll << 31), "rs_emb_forward: too many bags");
+    if (a.D <= 128) emb_fwd_sharded_kernel<1><<<static_cast<unsigned>(grid), wpb * 32, 0, stream>>>(a);
+    else if (a.D <= 256) emb_fwd_sharded_kernel<2><<<static_cast<unsigned>(grid), wpb * 32, 0, stream>>>(a);
+    else emb_fwd_sharded_kernel<4><<<static_cast<unsigned>(grid), wpb * 32, 0, stream>>>(a);
+    RS_LAUNCH_CHECK();
+    return RS_OK;
+  }
+  // How many bags share a sub-warp is settled on the device (it depends on the ids per bag); the host caps it so that a small
+  // batch still gives every SM sixteen warps, and sizes the grid for one-id bags: longer ones mean more tasks, over which
+  // the warps loop.
+  auto launch = [&](auto kern, int L) {
+    const int G = 32 / L;
+    int cap = L;
+    while (cap > 1 && bags / cap < 148ll * 16 * G) cap >>= 1;
+    const long long tasks = static_cast<long long>(a.T) * ((a.B + cap - 1) / cap);
+    long long grid = (tasks + wpb * G - 1) / (wpb * G);
+    if (per_sm > 0 && grid > 148ll * per_sm) grid = 148ll * per_sm;
+    kern<<<static_cast<unsigned>(grid), wpb * 32, 0, stream>>>(a, cap);
+  };
+#define RS_LAUNCH_POOL(V, L, NC) launch(emb_pool_kernel<V, L, NC>, L)
+  RS_ROW_DISPATCH(rs::row_wide(a.weight, a.D), a.D, RS_LAUNCH_POOL);
+#undef RS_LAUNCH_POOL
   RS_LAUNCH_CHECK();
   return RS_OK;
 }
@@ -688,27 +917,35 @@ int emb_backward_impl(float* weight, float* state, long long total_rows, const l
   a.B = B; a.D = D; a.grad_bf16 = grad_bf16;
   a.psw = psw; a.lr = lr; a.eps = eps; a.optimizer = optimizer; a.total_rows = total_rows; a.status = status;
   a.nnz_dev = nnz_dev; a.wait = wait;
-  const long long grid = (nnz + kGroup - 1) / kGroup;
-  RS_REQUIRE(grid < (1ll << 31), "rs_emb_backward: too many occurrences");
-  const int nc = D <= 128 ? 1 : (D <= 256 ? 2 : 4);
+  RS_REQUIRE(nnz < (1ll << 36), "rs_emb_backward: too many occurrences");
+  // 8-float units need rows and gradients that start on their boundaries (the offsets inside the gradient buffer are
+  // looked at in the kernel, they are device values).
+  const bool wide = rs::row_wide(weight, D) && (reinterpret_cast<uintptr_t>(grad) & (grad_bf16 ? 15 : 31)) == 0;
   if (optimizer == 1) {
-    const long long g1 = gnorm ? (nnz + 255) / 256 : (nnz + 7) / 8;
-    RS_REQUIRE(g1 < (1ll << 31), "rs_emb_backward: too many occurrences");
-    if (nc == 1) emb_state_kernel<1><<<static_cast<unsigned>(g1), 256, 0, stream>>>(a);
-    else if (nc == 2) emb_state_kernel<2><<<static_cast<unsigned>(g1), 256, 0, stream>>>(a);
-    else emb_state_kernel<4><<<static_cast<unsigned>(g1), 256, 0, stream>>>(a);
+    if (gnorm) {
+      emb_state_norm_kernel<<<static_cast<unsigned>((nnz + 255) / 256), 256, 0, stream>>>(a);
+    } else {
+      const int opw = nnz >= 32 * 8 * 148 ? 32 : 8;           // 32 occurrences per warp once every SM has eight warps
+      const unsigned g1 = static_cast<unsigned>((nnz + 8 * opw - 1) / (8 * opw));
+#define RS_LAUNCH_STATE(V, L, NC)                                                       \
+  do {                                                                                  \
+    if (grad_bf16) emb_state_kernel<V, L, NC, true><<<g1, 256, 0, stream>>>(a, opw);    \
+    else emb_state_kernel<V, L, NC, false><<<g1, 256, 0, stream>>>(a, opw);             \
+  } while (0)
+      RS_ROW_DISPATCH(wide, D, RS_LAUNCH_STATE);
+#undef RS_LAUNCH_STATE
+    }
     RS_LAUNCH_CHECK();
   }
-  const unsigned g = static_cast<unsigned>(grid);
-  if (grad_bf16) {
-    if (nc == 1) emb_apply_kernel<1, true><<<g, kGroup, 0, stream>>>(a);
-    else if (nc == 2) emb_apply_kernel<2, true><<<g, kGroup, 0, stream>>>(a);
-    else emb_apply_kernel<4, true><<<g, kGroup, 0, stream>>>(a);
-  } else {
-    if (nc == 1) emb_apply_kernel<1, false><<<g, kGroup, 0, stream>>>(a);
-    else if (nc == 2) emb_apply_kernel<2, false><<<g, kGroup, 0, stream>>>(a);
-    else emb_apply_kernel<4, false><<<g, kGroup, 0, stream>>>(a);
-  }
+  const int gs = nnz >= kGroup * 148 ? kGroup : 64;            // four times the CTAs while 256 per CTA would not fill the SMs
+  const unsigned g = static_cast<unsigned>((nnz + gs - 1) / gs);
+#define RS_LAUNCH_APPLY(V, L, NC)                                                          \
+  do {                                                                                     \
+    if (grad_bf16) emb_apply_kernel<V, L, NC, true><<<g, kGroup, 0, stream>>>(a, gs);      \
+    else emb_apply_kernel<V, L, NC, false><<<g, kGroup, 0, stream>>>(a, gs);               \
+  } while (0)
+  RS_ROW_DISPATCH(wide, D, RS_LAUNCH_APPLY);
+#undef RS_LAUNCH_APPLY
   RS_LAUNCH_CHECK();
   return RS_OK;
 }
