@@ -23,6 +23,7 @@
 #include "comm/flags.cuh"
 #include "common/rs_common.h"
 #include "kv/hash_table.cuh"
+#include "kv/key_init.cuh"
 
 namespace {
 
@@ -516,12 +517,7 @@ __global__ void __launch_bounds__(256) shard_keys_fused_kernel(const KeysFusedAr
   }
 }
 
-// Initial value of a row that the hash-table shard sees for the first time: uniform in [-scale, scale), a function of the key
-// and the column only, so a table does not depend on the order in which its keys arrive.
-__device__ __forceinline__ float key_init_value(unsigned long long key, int col, float scale) {
-  const unsigned long long h = rs::ht_hash(key * 0x9E3779B97F4A7C15ull + static_cast<unsigned long long>(col) + 1ull);
-  return (static_cast<float>(h >> 40) * (1.0f / 16777216.0f) * 2.f - 1.f) * scale;
-}
+using rs::key_init_value;
 
 struct GatherFusedArgs {
   float* weight;                    // local shard rows (HBM tier)

@@ -39,6 +39,7 @@ _lib.register_signatures({
     "rs_shard_gather_push_rows_tiered": (i32, [vp, vp, i64, i64, vp, vp, vp, vp, i32, i32, i32, i64, vp, vp]),
     "rs_tiered_apply": (i32, [vp, vp, vp, vp, i64, i64, vp, i64, i32, vp, vp, f32, f32, i32, vp]),
     "rs_rows_gather_checked": (i32, [vp, i64, vp, i64, i32, vp, vp, vp]),
+    "rs_shard_local": (i32, [vp, i64, vp, i64, i32, vp, vp, vp, vp, vp, C.POINTER(HashTableView), i32, i32, f32, vp, vp, vp]),
     "rs_shard_unbucket_rows": (i32, [vp, vp, i64, i32, vp, i32, vp]),
     "rs_shard_push_grads": (i32, [vp, vp, i64, i32, i32, i64, vp, vp, vp, vp]),
     "rs_segment_sum": (i32, [vp, vp, i64, i32, vp, vp, vp]),
@@ -155,6 +156,8 @@ class ShardedEmbeddingTable:
         self._grid_done = torch.zeros(4, dtype=torch.int32, device=dev)
         self._n = 0
         self.launches = 0
+        # One rank with its rows in HBM: every key is local, nothing is folded, bucketed or exchanged (csrc/kv/local_shard.cu).
+        self._local = self.world == 1 and not self.tiered and not self.range_c
 
     def close(self) -> None:
         """Collective: gives the five exchange windows back to the context (with a symmetric heap their bytes are reused
@@ -182,6 +185,11 @@ class ShardedEmbeddingTable:
         st, sp = self.ctx.status, stream_ptr()
         self._n = n
         self.launches = 0
+        if self._local:
+            if out is None:
+                out = torch.empty(n, self.D, device=self.dev)
+            self._local_verb(ids, n, st, sp, out=out, rows=self._occ_row)
+            return out
         if self.dedup:
             self._uniq[:n].fill_(-1)
             _lib.call("rs_unique_keys", ptr(ids), n, ptr(self._sk), ptr(self._si), self._nslots, ptr(self._uniq), ptr(self._inv),
@@ -190,18 +198,6 @@ class ShardedEmbeddingTable:
             self.launches += 3
         else:
             keys = ids
-        if self.world == 1 and not self.tiered and not self.hashed and not self.range_c:
-            # One rank: every row is local (local row = id), so nothing is bucketed or exchanged.
-            src_keys = keys[:n]
-            if out is None:
-                out = torch.empty(n, self.D, device=self.dev)
-            dst = self._urows if self.dedup else out
-            _lib.call("rs_rows_gather_checked", ptr(self.weight), self.N, ptr(src_keys), n, self.D, ptr(dst), ptr(st), sp)
-            if self.dedup:
-                _lib.call("rs_expand_rows", ptr(self._urows), ptr(self._inv), n, self.D, ptr(out), sp)
-            self._local_rows = src_keys
-            self.launches += 2
-            return out
         if self.fused:
             return self._lookup_fused(keys, n, out, st, sp)
         _lib.call("rs_shard_push_keys", ptr(keys), n, self.world, self.rank, self.cap, ptr(self._counts), ptr(self._cursor),
@@ -225,6 +221,19 @@ class ShardedEmbeddingTable:
             _lib.call("rs_shard_unbucket_rows", self.row_win.local_ptr, ptr(self._slot), n, self.D, ptr(out), 0, sp)
         self.launches += 9
         return out
+
+    def _local_verb(self, ids, n, st, sp, out=None, rows=None, found=None, values=None, state=None, find_only=False, folded=None):
+        """One launch for any verb of a one-rank shard; ``rows`` receives the row of every id for the update to come."""
+        folded = self.dedup if folded is None else folded
+        _lib.call("rs_shard_local", ptr(self.weight), self.local_rows, ptr(ids), n, self.D, ptr(out), ptr(rows), ptr(found), ptr(values),
+                  ptr(state), C.byref(self._ht_view) if self.hashed else None, 1 if find_only else 0, 1 if folded else 0,
+                  self.init_scale, ptr(self.row_init) if self.hashed else None, ptr(st), sp)
+        self.launches += 1
+
+    def _local_update(self, grads, n, st, norms=None):
+        F_.emb_backward(self.weight, self.state, self._occ_row, None, n, grads, grad_row_stride=self.D, B=max(n, 1) if self.hashed else n,
+                        D=self.D, grad_bf16=False, lr=self.lr, eps=self.eps, optimizer=self.optimizer, status=st, gnorm=norms, gnorm_stride=1)
+        self.launches += 2 if self.optimizer == "rowwise_adagrad" else 1
 
     def _lookup_fused(self, keys, n, out, st, sp):
         c = self.ctx
@@ -266,8 +275,12 @@ class ShardedEmbeddingTable:
         n = ids.numel()
         assert n <= self.world * self.cap
         st, sp = self.ctx.status, stream_ptr()
-        self._exchange_keys(ids, n, st, sp, push_rows=True, find_only=self.hashed, folded=False)
         out = torch.empty(n, self.D, device=self.dev)
+        if self._local:
+            found = torch.empty(n, dtype=torch.bool, device=self.dev)
+            self._local_verb(ids, n, st, sp, out=out, found=found, find_only=self.hashed, folded=False)
+            return out, found
+        self._exchange_keys(ids, n, st, sp, push_rows=True, find_only=self.hashed, folded=False)
         c = self.ctx
         _lib.call("rs_shard_unbucket_fused", self.row_win.local_ptr, ptr(self._slot), None, n, self.D, ptr(out), 0, None, None, None,
                   ptr(ids), None, 0, c.my_flags_ptr, c.counters_ptr, c.wait_timeout_ns, CH_ROWS, self.world, ptr(st), sp)
@@ -283,6 +296,9 @@ class ShardedEmbeddingTable:
         n = ids.numel()
         assert n <= self.world * self.cap and values.shape == (n, self.D) and values.dtype == torch.float32
         st, sp, c = self.ctx.status, stream_ptr(), self.ctx
+        if self._local:
+            self._local_verb(ids, n, st, sp, values=values, state=self.state, folded=False)
+            return
         self._exchange_keys(ids, n, st, sp, push_rows=False, folded=False)
         _lib.call("rs_shard_grads_fused", ptr(values), ptr(self._slot), None, n, self.D, self.rank, self.cap, ptr(self.grad_win.table),
                   None, None, c.flags_table_ptr, c.counters_ptr, ptr(self._grid_done[2:3]), CH_GRADS, self.world, sp)
@@ -310,6 +326,10 @@ class ShardedEmbeddingTable:
         st, sp = self.ctx.status, stream_ptr()
         self._n = n
         self.launches = 0
+        if self._local:
+            self._local_verb(ids, n, st, sp, rows=self._occ_row)
+            self._local_update(grads, n, st)
+            return
         if self.dedup:
             _lib.call("rs_unique_keys", ptr(ids), n, ptr(self._sk), ptr(self._si), self._nslots, ptr(self._uniq), ptr(self._inv),
                       ptr(self._ucount), ptr(st), sp)
@@ -367,18 +387,9 @@ class ShardedEmbeddingTable:
         assert norms is None or self.dedup, "per-occurrence norms need a deduplicating table"
         grads = grads.contiguous()
         st, sp = self.ctx.status, stream_ptr()
-        if self.world == 1 and not self.tiered and not self.hashed and not self.range_c:
-            if self.dedup:
-                self._ugrad[:n].zero_()
-                self._unorm[:n].zero_()
-                self._fold(grads, n, sp, norms)
-                g, gn = self._ugrad, self._unorm
-            else:
-                g, gn = grads, None
-            F_.emb_backward(self.weight, self.state, self._local_rows, None, n, g, grad_row_stride=self.D, B=n, D=self.D,
-                            grad_bf16=False, lr=self.lr, eps=self.eps, optimizer=self.optimizer, status=st, gnorm=gn, gnorm_stride=1)
-            self.launches += 5
-            return
+        if self._local:
+            assert norms is None or (norms.numel() == n and norms.dtype == torch.float32 and norms.is_contiguous())
+            return self._local_update(grads, n, st, norms)
         if self.fused:
             return self._update_fused(grads, n, st, sp, norms)
         gnorm = None
