@@ -439,8 +439,9 @@ __device__ __forceinline__ long long live_nnz(const EmbBwdArgs& a) {
   return n < a.nnz ? n : a.nnz;
 }
 
-constexpr int kGroup = 256;      // threads of an apply CTA, and the most occurrences it takes
-constexpr int kSlots = 2 * kGroup;
+constexpr int kStateMax = 1024;  // occurrences a CTA of the state pass folds
+constexpr int kApplyThreads = 512;
+constexpr int kApplyMax = 1024;  // occurrences a CTA of the apply pass sorts
 
 // Sample and table of occurrence i.  32-bit arithmetic wherever the bag number allows it: a 64-bit division costs more
 // than the rest of the address computation.
@@ -459,117 +460,170 @@ __device__ __forceinline__ void bag_of(const EmbBwdArgs& a, long long i, int& t,
 }
 
 // Pass 1 of row-wise Adagrad: state[row] += w^2 * |g_bag|^2 / D for every occurrence.
-// With precomputed bag norms it is one thread per occurrence; the lanes of a warp that hold the same row add up in
-// registers first, so a warp sends one atomic per distinct row.  Bound by the issue of the chain steps and by the scattered
-// 4-byte norms.  It replaced a shared-memory hash whose float adds are compare-and-swap loops that the hot rows of a skewed
-// id stream serialise: 1.70 M occurrences at Zipf 1.2 took 49 us.
-__global__ void __launch_bounds__(256) emb_state_norm_kernel(const EmbBwdArgs a) {
-  const long long nnz = live_nnz(a);
-  if (static_cast<long long>(blockIdx.x) * blockDim.x >= nnz) return;   // whole block past the live occurrences
-  rs::flag_wait_all(a.wait);
-  const float inv_d = 1.f / static_cast<float>(a.D);
-  const long long i = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x;
-  long long row = -1;
-  float v = 0.f;
-  if (i < nnz) {
-    row = a.row_idx[i];
-    if (row < 0 || row >= a.total_rows) {
-      row = -1;
-    } else {
-      int t, b;
-      bag_of(a, i, t, b);
-      const float w = a.psw ? a.psw[i] : 1.f;
-      v = w * w * a.gnorm[static_cast<long long>(b) * a.gnorm_stride + t] * inv_d;
-    }
+// A CTA folds up to 1,024 occurrences before it touches the state: the lanes of a warp that hold the same row add up in
+// registers, one lane per row and warp adds to a shared-memory hash, and one global atomic per distinct row of the CTA
+// follows.  Without the first fold the float adds in shared memory, compare-and-swap loops, are serialised by the hot rows of
+// a skewed id stream (49 us for 1.70 M occurrences at Zipf 1.2); without the second the global atomics on the hottest row are
+// (33 us for 262,144 occurrences at Zipf 1.1), and its sum becomes a chain of thousands of fp32 roundings.
+struct StateFold {
+  unsigned long long key[2 * kStateMax];
+  float val[2 * kStateMax];
+};
+__device__ __forceinline__ void state_fold_clear(StateFold& f, int slots) {
+  for (int s = threadIdx.x; s < slots; s += blockDim.x) {
+    f.key[s] = ~0ull;
+    f.val[s] = 0.f;
   }
+  __syncthreads();
+}
+// All lanes of a warp; row < 0: nothing to add.
+__device__ __forceinline__ void state_fold_add(StateFold& f, int slots, long long row, float v) {
   const bool first = rs::warp_sum_equal_keys(static_cast<unsigned long long>(row), v);
-  if (first && row >= 0) atomicAdd(&a.state[row], v);
+  if (!first || row < 0) return;
+  unsigned s = static_cast<unsigned>(rs::ht_hash(static_cast<unsigned long long>(row))) & (slots - 1);
+  for (int p = 0; p < slots; ++p) {
+    const unsigned long long prev = atomicCAS(&f.key[s], ~0ull, static_cast<unsigned long long>(row));
+    if (prev == ~0ull || prev == static_cast<unsigned long long>(row)) {
+      atomicAdd(&f.val[s], v);
+      return;
+    }
+    s = (s + 1) & (slots - 1);
+  }
+}
+__device__ __forceinline__ void state_fold_flush(const StateFold& f, int slots, float* state) {
+  __syncthreads();
+  for (int s = threadIdx.x; s < slots; s += blockDim.x)
+    if (f.key[s] != ~0ull) atomicAdd(&state[f.key[s]], f.val[s]);
 }
 
-// Without norms a warp takes `opw` consecutive occurrences (32, or 8 when the batch would leave SMs without work): its
-// sub-warps compute the squared norms, U gradient rows of each in flight, and the lanes then add up as above.
-template <int V, int L, int NC, bool BF16>
-__global__ void __launch_bounds__(256) emb_state_kernel(const EmbBwdArgs a, const int opw) {
-  constexpr int G = 32 / L;
-  constexpr int U = V * NC <= 8 ? 4 : 2;
+// With precomputed bag norms: one thread per occurrence, `rounds` (at most 4) of them per thread.
+__global__ void __launch_bounds__(256) emb_state_norm_kernel(const EmbBwdArgs a, const int rounds) {
+  __shared__ StateFold f;
   const long long nnz = live_nnz(a);
-  const long long i0 = (static_cast<long long>(blockIdx.x) * (blockDim.x >> 5) + (threadIdx.x >> 5)) * opw;
-  if (static_cast<long long>(blockIdx.x) * (blockDim.x >> 5) * opw >= nnz) return;
+  const long long i0 = static_cast<long long>(blockIdx.x) * 256 * rounds;
+  if (i0 >= nnz) return;                       // whole block past the live occurrences
   rs::flag_wait_all(a.wait);
-  const int lane = threadIdx.x & 31, l = lane & (L - 1), g = lane / L;
-  const long long i = i0 + lane;
-  long long row = -1, goff = 0;
-  float w = 1.f, v = 0.f;
-  if (lane < opw && i < nnz) {
-    row = a.row_idx[i];
-    if (row >= a.total_rows) row = -1;
-    if (row >= 0) {
-      int t, b;
-      bag_of(a, i, t, b);
-      goff = b * a.grad_row_stride + (a.grad_col ? a.grad_col[t] : 0);
-      if (a.psw) w = a.psw[i];
-    } else {
-      row = -1;
-    }
-  }
-  const bool wide = V == 4 || __all_sync(0xffffffffu, (goff & 7) == 0);
-  const int nvec = a.D / V;
-  for (int j0 = 0; j0 < opw; j0 += G * U) {
-    rs::RawVec<V, BF16> x[U][NC];
-    bool on[U];
+  const int slots = 512 * rounds;
+  state_fold_clear(f, slots);
+  const float inv_d = 1.f / static_cast<float>(a.D);
+  long long row[4];
+  float v[4];
 #pragma unroll
-    for (int u = 0; u < U; ++u) {
-      const int j = (j0 + u * G + g) & 31;
-      const long long go = __shfl_sync(0xffffffffu, goff, j);
-      on[u] = __shfl_sync(0xffffffffu, row, j) >= 0 && j0 + u * G + g < opw;
-      if (on[u]) {
-#pragma unroll
-        for (int c = 0; c < NC; ++c) x[u][c].load(a.grad, go + static_cast<long long>(min(l + c * L, nvec - 1)) * V, wide);
+  for (int r = 0; r < 4; ++r) {
+    const long long i = i0 + r * 256 + threadIdx.x;
+    row[r] = -1;
+    v[r] = 0.f;
+    if (r < rounds && i < nnz) {
+      row[r] = a.row_idx[i];
+      if (row[r] < 0 || row[r] >= a.total_rows) {
+        row[r] = -1;
+      } else {
+        int t, b;
+        bag_of(a, i, t, b);
+        const float w = a.psw ? a.psw[i] : 1.f;
+        v[r] = w * w * a.gnorm[static_cast<long long>(b) * a.gnorm_stride + t] * inv_d;
       }
     }
+  }
 #pragma unroll
-    for (int u = 0; u < U; ++u) {
-      float sq = 0.f;
-      if (on[u]) {
+  for (int r = 0; r < 4; ++r)
+    if (r < rounds) state_fold_add(f, slots, row[r], v[r]);
+  state_fold_flush(f, slots, a.state);
+}
+
+// Without norms a warp takes `opw` consecutive occurrences per round (32, fewer when the batch would leave SMs without work):
+// its sub-warps compute the squared norms, U gradient rows of each in flight.
+template <int V, int L, int NC, bool BF16>
+__global__ void __launch_bounds__(256) emb_state_kernel(const EmbBwdArgs a, const int opw, const int rounds) {
+  constexpr int G = 32 / L;
+  constexpr int U = V * NC <= 8 ? 4 : 2;
+  __shared__ StateFold f;
+  const long long nnz = live_nnz(a);
+  const long long c0 = static_cast<long long>(blockIdx.x) * 8 * opw * rounds;
+  if (c0 >= nnz) return;
+  rs::flag_wait_all(a.wait);
+  const int slots = 16 * opw * rounds;
+  state_fold_clear(f, slots);
+  const int lane = threadIdx.x & 31, l = lane & (L - 1), g = lane / L;
+  const int nvec = a.D / V;
+  for (int rd = 0; rd < rounds; ++rd) {
+    const long long i = c0 + (rd * 8 + (threadIdx.x >> 5)) * opw + lane;
+    long long row = -1, goff = 0;
+    float w = 1.f, v = 0.f;
+    if (lane < opw && i < nnz) {
+      row = a.row_idx[i];
+      if (row < 0 || row >= a.total_rows) {
+        row = -1;
+      } else {
+        int t, b;
+        bag_of(a, i, t, b);
+        goff = b * a.grad_row_stride + (a.grad_col ? a.grad_col[t] : 0);
+        if (a.psw) w = a.psw[i];
+      }
+    }
+    const bool wide = V == 4 || __all_sync(0xffffffffu, (goff & 7) == 0);
+    for (int j0 = 0; j0 < opw; j0 += G * U) {
+      rs::RawVec<V, BF16> x[U][NC];
+      bool on[U];
 #pragma unroll
-        for (int c = 0; c < NC; ++c) {
-          if (l + c * L < nvec) {
-            const rs::RowVec<V> f = x[u][c].get();
+      for (int u = 0; u < U; ++u) {
+        const int j = (j0 + u * G + g) & 31;
+        const long long go = __shfl_sync(0xffffffffu, goff, j);
+        on[u] = __shfl_sync(0xffffffffu, row, j) >= 0 && j0 + u * G + g < opw;
+        if (on[u]) {
 #pragma unroll
-            for (int e = 0; e < V; ++e) sq += f.v[e] * f.v[e];
-          }
+          for (int c = 0; c < NC; ++c) x[u][c].load(a.grad, go + static_cast<long long>(min(l + c * L, nvec - 1)) * V, wide);
         }
       }
 #pragma unroll
-      for (int o = L / 2; o > 0; o >>= 1) sq += __shfl_xor_sync(0xffffffffu, sq, o);
-      // occurrence j0 + u * G + k lies in sub-warp k; lane j keeps the norm of occurrence j
-      const int k = lane - j0 - u * G;
-      const float got = __shfl_sync(0xffffffffu, sq, (k & (G - 1)) * L);
-      if (k >= 0 && k < G) v = got;
+      for (int u = 0; u < U; ++u) {
+        float sq = 0.f;
+        if (on[u]) {
+#pragma unroll
+          for (int c = 0; c < NC; ++c) {
+            if (l + c * L < nvec) {
+              const rs::RowVec<V> h = x[u][c].get();
+#pragma unroll
+              for (int e = 0; e < V; ++e) sq += h.v[e] * h.v[e];
+            }
+          }
+        }
+#pragma unroll
+        for (int o = L / 2; o > 0; o >>= 1) sq += __shfl_xor_sync(0xffffffffu, sq, o);
+        // occurrence j0 + u * G + k lies in sub-warp k; lane j keeps the norm of occurrence j
+        const int k = lane - j0 - u * G;
+        const float got = __shfl_sync(0xffffffffu, sq, (k & (G - 1)) * L);
+        if (k >= 0 && k < G) v = got;
+      }
     }
+    v *= w * w / static_cast<float>(a.D);
+    state_fold_add(f, slots, row, v);
   }
-  v *= w * w / static_cast<float>(a.D);
-  const bool first = rs::warp_sum_equal_keys(static_cast<unsigned long long>(row), v);
-  if (first && row >= 0) atomicAdd(&a.state[row], v);
+  state_fold_flush(f, slots, a.state);
 }
 
-// Apply pass: one CTA per `gs` occurrences (256, or 64 when that leaves SMs without work).  They are counting-sorted by row
+// Apply pass: one CTA per `gs` occurrences (1,024 at most, fewer when that leaves SMs without work).  They are counting-sorted by row
 // in shared memory (hash slot -> count -> exclusive scan -> position), so equal rows sit next to each other, together with
 // their factor -lr * w / (sqrt(state) + eps): one state read and one root per occurrence, by the thread that owns it, and
 // none in the loop over the rows.  Every sub-warp then owns an equal share of the sorted positions, whatever the skew of the
 // ids: it streams their gradients with U loads in flight, sums runs of equal rows in registers and issues one vector
-// atomic per unit and run.  A row that straddles sub-warps or groups simply receives several atomics.
-// Bound by issue slots and latency: 16-byte bf16 loads by half a warp per 128-float row, at four or five CTAs per SM.  The
-// form before it (a warp per row, state read and root inside the loop, 76 registers, 32 % of the warps resident) took
+// atomic per unit and run.  A row that straddles warps or groups simply receives several atomics; the larger the group the
+// fewer of them meet on the hot rows, which the L2 takes one after another.
+// Bound by latency (sort, then gradients) and by those atomics: 16-byte bf16 loads by half a warp per 128-float row.  The
+// form before it (256 occurrences, a warp per row, state read and root inside the loop, 32 % of the warps resident) took
 // 278 us for 1.70 M occurrences x 128 at Zipf 1.2.
 template <int V, int L, int NC, bool BF16>
-__global__ void __launch_bounds__(kGroup) emb_apply_kernel(const EmbBwdArgs a, const int gs) {
-  __shared__ long long s_key[kSlots];
-  __shared__ int s_cnt[kSlots];         // occurrences per slot, then exclusive offsets
-  __shared__ long long s_goff[kGroup];  // sorted: gradient offset
-  __shared__ long long s_row[kGroup];   // sorted: row
-  __shared__ float s_coef[kGroup];      // sorted: factor of the gradient
-  __shared__ int s_warp_sum[kGroup / 32];
+__global__ void __launch_bounds__(kApplyThreads) emb_apply_kernel(const EmbBwdArgs a, const int gs) {
+  constexpr int kPer = kApplyMax / kApplyThreads;
+  constexpr int kWarps = kApplyThreads / 32;
+  // the hash is dead once the positions are known; the sorted arrays take its place
+  __shared__ __align__(16) unsigned char s_mem[2 * kApplyMax * 12 > kApplyMax * 20 ? 2 * kApplyMax * 12 : kApplyMax * 20];
+  __shared__ int s_warp_sum[kWarps];
+  long long* const s_key = reinterpret_cast<long long*>(s_mem);                        // [2 gs]
+  int* const s_cnt = reinterpret_cast<int*>(s_mem + 2 * kApplyMax * 8);                // [2 gs] occurrences per slot, then offsets
+  long long* const s_goff = reinterpret_cast<long long*>(s_mem);                       // sorted: gradient offset
+  long long* const s_row = reinterpret_cast<long long*>(s_mem + kApplyMax * 8);        // sorted: row
+  float* const s_coef = reinterpret_cast<float*>(s_mem + kApplyMax * 16);              // sorted: factor of the gradient
 
   const int tid = threadIdx.x;
   const int warp = tid >> 5, lane = tid & 31;
@@ -578,49 +632,70 @@ __global__ void __launch_bounds__(kGroup) emb_apply_kernel(const EmbBwdArgs a, c
   if (g0 >= nnz) return;                       // whole group past the live occurrences
   rs::flag_wait_all(a.wait);
   const int slots = 2 * gs;
-  for (int s = tid; s < slots; s += kGroup) {
+  for (int s = tid; s < slots; s += kApplyThreads) {
     s_key[s] = -1;
     s_cnt[s] = 0;
   }
-  long long row = -1, goff = 0;
-  float coef = -a.lr;
-  int slot = -1, rank = 0;
-  if (tid < gs && g0 + tid < nnz) {
-    const long long occ = g0 + tid;
-    row = a.row_idx[occ];
-    if (row >= a.total_rows) {
-      if (a.status) atomicOr(a.status, (unsigned long long)RS_DEV_OOB_ROW);
-      row = -1;
-    }
-    if (row >= 0) {
-      int t, b;
-      bag_of(a, occ, t, b);
-      goff = b * a.grad_row_stride + (a.grad_col ? a.grad_col[t] : 0);
-      if (a.optimizer == 1) coef = -a.lr / (sqrtf(__ldcv(&a.state[row])) + a.eps);
-      if (a.psw) coef *= a.psw[occ];
+  long long row[kPer], goff[kPer];
+  float coef[kPer];
+  bool narrow = false;
+#pragma unroll
+  for (int q = 0; q < kPer; ++q) {
+    const int at = q * kApplyThreads + tid;
+    row[q] = -1;
+    goff[q] = 0;
+    coef[q] = -a.lr;
+    if (at < gs && g0 + at < nnz) {
+      row[q] = a.row_idx[g0 + at];
+      if (row[q] >= a.total_rows) {
+        if (a.status) atomicOr(a.status, (unsigned long long)RS_DEV_OOB_ROW);
+        row[q] = -1;
+      }
     }
   }
-  const bool wide = !__syncthreads_or(V == 8 && (goff & 7) != 0);   // (also: the slots are cleared)
-  if (row >= 0) {
-    unsigned s = static_cast<unsigned>(rs::ht_hash(static_cast<unsigned long long>(row))) & (slots - 1);
+#pragma unroll
+  for (int q = 0; q < kPer; ++q) {
+    if (row[q] < 0) continue;
+    const long long occ = g0 + q * kApplyThreads + tid;
+    int t, b;
+    bag_of(a, occ, t, b);
+    goff[q] = b * a.grad_row_stride + (a.grad_col ? a.grad_col[t] : 0);
+    if (a.optimizer == 1) coef[q] = -a.lr / (sqrtf(__ldcv(&a.state[row[q]])) + a.eps);
+    if (a.psw) coef[q] *= a.psw[occ];
+    narrow = narrow || (goff[q] & 7) != 0;
+  }
+  const bool wide = !__syncthreads_or(V == 8 && narrow);   // (also: the slots are cleared)
+  int slot[kPer], rank[kPer];
+#pragma unroll
+  for (int q = 0; q < kPer; ++q) {
+    slot[q] = -1;
+    rank[q] = 0;
+    if (row[q] < 0) continue;
+    unsigned s = static_cast<unsigned>(rs::ht_hash(static_cast<unsigned long long>(row[q]))) & (slots - 1);
     for (int p = 0; p < slots; ++p) {
       const long long prev = static_cast<long long>(atomicCAS(reinterpret_cast<unsigned long long*>(&s_key[s]),
                                                                static_cast<unsigned long long>(-1ll),
-                                                               static_cast<unsigned long long>(row)));
-      if (prev == -1 || prev == row) {
-        slot = static_cast<int>(s);
-        rank = atomicAdd(&s_cnt[s], 1);
+                                                               static_cast<unsigned long long>(row[q])));
+      if (prev == -1 || prev == row[q]) {
+        slot[q] = static_cast<int>(s);
+        rank[q] = atomicAdd(&s_cnt[s], 1);
         break;
       }
       s = (s + 1) & (slots - 1);
     }
   }
   __syncthreads();
-  // exclusive scan of the slot counts: two slots per thread, warp shuffles, then the warp totals
+  // exclusive scan of the slot counts: 2 * kPer neighbouring slots per thread, warp shuffles, then the warp totals
+  int total = 0;
   {
-    const bool mine = 2 * tid < slots;
-    const int c0 = mine ? s_cnt[2 * tid] : 0, c1 = mine ? s_cnt[2 * tid + 1] : 0;
-    int incl = c0 + c1;
+    constexpr int kScan = 2 * kPer;
+    int c[kScan], sum = 0;
+#pragma unroll
+    for (int q = 0; q < kScan; ++q) {
+      c[q] = kScan * tid + q < slots ? s_cnt[kScan * tid + q] : 0;
+      sum += c[q];
+    }
+    int incl = sum;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
       const int y = __shfl_up_sync(0xffffffffu, incl, o);
@@ -628,32 +703,37 @@ __global__ void __launch_bounds__(kGroup) emb_apply_kernel(const EmbBwdArgs a, c
     }
     if (lane == 31) s_warp_sum[warp] = incl;
     __syncthreads();
-    int base = 0;
+    int excl = incl - sum;
 #pragma unroll
-    for (int q = 0; q < kGroup / 32; ++q) base += q < warp ? s_warp_sum[q] : 0;
-    const int excl = base + incl - (c0 + c1);
-    if (mine) {
-      s_cnt[2 * tid] = excl;
-      s_cnt[2 * tid + 1] = excl + c0;
+    for (int q = 0; q < kWarps; ++q) {
+      excl += q < warp ? s_warp_sum[q] : 0;
+      total += s_warp_sum[q];
+    }
+#pragma unroll
+    for (int q = 0; q < kScan; ++q) {
+      if (kScan * tid + q < slots) s_cnt[kScan * tid + q] = excl;
+      excl += c[q];
     }
   }
   __syncthreads();
-  if (slot >= 0) {
-    const int pos = s_cnt[slot] + rank;
-    s_goff[pos] = goff;
-    s_row[pos] = row;
-    s_coef[pos] = coef;
+  int pos[kPer];
+#pragma unroll
+  for (int q = 0; q < kPer; ++q) pos[q] = slot[q] >= 0 ? s_cnt[slot[q]] + rank[q] : -1;
+  __syncthreads();                              // the hash has been read for the last time
+#pragma unroll
+  for (int q = 0; q < kPer; ++q) {
+    if (pos[q] < 0) continue;
+    s_goff[pos[q]] = goff[q];
+    s_row[pos[q]] = row[q];
+    s_coef[pos[q]] = coef[q];
   }
   __syncthreads();
 
   constexpr int G = 32 / L;
   constexpr int U = V * NC <= 8 ? 4 : 2;
-  int total = 0;
-#pragma unroll
-  for (int q = 0; q < kGroup / 32; ++q) total += s_warp_sum[q];
   const int l = lane & (L - 1);
   const int nvec = a.D / V;
-  const int share = gs / ((kGroup / 32) * G);
+  const int share = gs / (kWarps * G);
   const int p_begin = (warp * G + lane / L) * share;
   const int p_end = min(total, p_begin + share);
   long long cur = -1;
@@ -690,15 +770,15 @@ __global__ void __launch_bounds__(kGroup) emb_apply_kernel(const EmbBwdArgs a, c
       const float k = s_coef[p0 + u];
 #pragma unroll
       for (int c = 0; c < NC; ++c) {
-        const rs::RowVec<V> f = x[u][c].get();
+        const rs::RowVec<V> h = x[u][c].get();
 #pragma unroll
-        for (int e = 0; e < V; ++e) acc[c].v[e] = fmaf(k, f.v[e], acc[c].v[e]);
+        for (int e = 0; e < V; ++e) acc[c].v[e] = fmaf(k, h.v[e], acc[c].v[e]);
       }
     }
   }
   if (G > 1) {
     // A hot row fills whole sub-warps: equal rows at the ends of neighbouring sub-warps are added up towards the first of
-    // them, which alone sends (a 32-float row has eight sub-warps of four positions each, and as many atomics otherwise).
+    // them, which alone sends.
     __syncwarp();
 #pragma unroll
     for (int o = 1; o < G; o <<= 1) {
@@ -708,8 +788,8 @@ __global__ void __launch_bounds__(kGroup) emb_apply_kernel(const EmbBwdArgs a, c
       for (int c = 0; c < NC; ++c)
 #pragma unroll
         for (int e = 0; e < V; ++e) {
-          const float x = __shfl_down_sync(0xffffffffu, acc[c].v[e], o * L);
-          if (join) acc[c].v[e] += x;
+          const float y = __shfl_down_sync(0xffffffffu, acc[c].v[e], o * L);
+          if (join) acc[c].v[e] += y;
         }
     }
     const long long before = __shfl_up_sync(0xffffffffu, cur, L);
@@ -922,27 +1002,36 @@ int emb_backward_impl(float* weight, float* state, long long total_rows, const l
   // looked at in the kernel, they are device values).
   const bool wide = rs::row_wide(weight, D) && (reinterpret_cast<uintptr_t>(grad) & (grad_bf16 ? 15 : 31)) == 0;
   if (optimizer == 1) {
+    // As many occurrences per CTA as keep every SM busy with two CTAs, 1,024 at most.
     if (gnorm) {
-      emb_state_norm_kernel<<<static_cast<unsigned>((nnz + 255) / 256), 256, 0, stream>>>(a);
+      const int rounds = nnz >= 1024 * 296 ? 4 : nnz >= 512 * 296 ? 2 : 1;
+      emb_state_norm_kernel<<<static_cast<unsigned>((nnz + 256 * rounds - 1) / (256 * rounds)), 256, 0, stream>>>(a, rounds);
     } else {
-      const int opw = nnz >= 32 * 8 * 148 ? 32 : 8;           // 32 occurrences per warp once every SM has eight warps
-      const unsigned g1 = static_cast<unsigned>((nnz + 8 * opw - 1) / (8 * opw));
-#define RS_LAUNCH_STATE(V, L, NC)                                                       \
-  do {                                                                                  \
-    if (grad_bf16) emb_state_kernel<V, L, NC, true><<<g1, 256, 0, stream>>>(a, opw);    \
-    else emb_state_kernel<V, L, NC, false><<<g1, 256, 0, stream>>>(a, opw);             \
+      auto launch = [&](auto kern, int L) {
+        int opw = 32, rounds = nnz >= 1024 * 296 ? 4 : nnz >= 512 * 296 ? 2 : 1;
+        while (opw > 32 / L && nnz < 8ll * opw * 296) opw >>= 1;
+        kern<<<static_cast<unsigned>((nnz + 8 * opw * rounds - 1) / (8 * opw * rounds)), 256, 0, stream>>>(a, opw, rounds);
+      };
+#define RS_LAUNCH_STATE(V, L, NC)                                 \
+  do {                                                            \
+    if (grad_bf16) launch(emb_state_kernel<V, L, NC, true>, L);   \
+    else launch(emb_state_kernel<V, L, NC, false>, L);            \
   } while (0)
       RS_ROW_DISPATCH(wide, D, RS_LAUNCH_STATE);
 #undef RS_LAUNCH_STATE
     }
     RS_LAUNCH_CHECK();
   }
-  const int gs = nnz >= kGroup * 148 ? kGroup : 64;            // four times the CTAs while 256 per CTA would not fill the SMs
-  const unsigned g = static_cast<unsigned>((nnz + gs - 1) / gs);
-#define RS_LAUNCH_APPLY(V, L, NC)                                                          \
-  do {                                                                                     \
-    if (grad_bf16) emb_apply_kernel<V, L, NC, true><<<g, kGroup, 0, stream>>>(a, gs);      \
-    else emb_apply_kernel<V, L, NC, false><<<g, kGroup, 0, stream>>>(a, gs);               \
+  // The largest group that still gives every SM two CTAs, never less than one position per sub-warp.
+  auto launch = [&](auto kern, int L) {
+    int gs = kApplyMax;
+    while (gs > (kApplyThreads / 32) * (32 / L) && nnz < 296ll * gs) gs >>= 1;
+    kern<<<static_cast<unsigned>((nnz + gs - 1) / gs), kApplyThreads, 0, stream>>>(a, gs);
+  };
+#define RS_LAUNCH_APPLY(V, L, NC)                                 \
+  do {                                                            \
+    if (grad_bf16) launch(emb_apply_kernel<V, L, NC, true>, L);   \
+    else launch(emb_apply_kernel<V, L, NC, false>, L);            \
   } while (0)
   RS_ROW_DISPATCH(wide, D, RS_LAUNCH_APPLY);
 #undef RS_LAUNCH_APPLY
