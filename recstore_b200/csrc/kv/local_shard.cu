@@ -36,7 +36,7 @@ __device__ __forceinline__ void load_16(rs::RowVec<8>& r, const float* p) {
 }
 __device__ __forceinline__ void load_16(rs::RowVec<4>& r, const float* p) { rs::row_load_nc(r, p); }
 
-// A warp takes `kpw` consecutive ids (32, or 8 when the batch would leave SMs without work).  Every lane resolves one of them, so
+// A warp takes `kpw` consecutive ids (32, fewer when the batch would leave SMs without work).  Every lane resolves one of them, so
 // up to 32 hash probes are in flight per warp; its sub-warps of L lanes then copy the rows, U of them in flight each.
 template <int V, int L>
 __global__ void __launch_bounds__(128) local_shard_kernel(const LocalShardArgs a, const int kpw) {
@@ -170,19 +170,26 @@ RS_API int rs_shard_local(float* weight, long long local_rows, const long long* 
   a.values = values; a.state = state; a.use_hash = ht != nullptr; a.find_only = find_only; a.refuse_reserved = refuse_reserved;
   if (ht) a.ht = *ht;
   a.init_scale = init_scale; a.row_init = row_init; a.status = status;
-  const int kpw = n >= 32 * 16 * 148 ? 32 : 8;         // 32 ids per warp once every SM has sixteen warps
-  const long long grid = (n + 4 * kpw - 1) / (4 * kpw);
-  RS_REQUIRE(grid < (1ll << 31), "rs_shard_local: too many ids");
-  const unsigned g = static_cast<unsigned>(grid);
+  // Ids per warp: 32 once every SM has sixteen warps, fewer in a small batch, but one for every sub-warp.
+  auto launch = [&](auto kern, int L) -> int {
+    int kpw = 32;
+    while (kpw > 32 / L && n < 148ll * 16 * kpw) kpw >>= 1;
+    const long long grid = (n + 4 * kpw - 1) / (4 * kpw);
+    RS_REQUIRE(grid < (1ll << 31), "rs_shard_local: too many ids");
+    kern<<<static_cast<unsigned>(grid), 128, 0, stream>>>(a, kpw);
+    return RS_OK;
+  };
+  int rc;
   if (rs::row_wide(weight, D)) {
-    if (D <= 32) local_shard_kernel<8, 4><<<g, 128, 0, stream>>>(a, kpw);
-    else if (D <= 64) local_shard_kernel<8, 8><<<g, 128, 0, stream>>>(a, kpw);
-    else if (D <= 128) local_shard_kernel<8, 16><<<g, 128, 0, stream>>>(a, kpw);
-    else local_shard_kernel<8, 32><<<g, 128, 0, stream>>>(a, kpw);
+    if (D <= 32) rc = launch(local_shard_kernel<8, 4>, 4);
+    else if (D <= 64) rc = launch(local_shard_kernel<8, 8>, 8);
+    else if (D <= 128) rc = launch(local_shard_kernel<8, 16>, 16);
+    else rc = launch(local_shard_kernel<8, 32>, 32);
   } else {
-    if (D <= 32) local_shard_kernel<4, 8><<<g, 128, 0, stream>>>(a, kpw);
-    else local_shard_kernel<4, 32><<<g, 128, 0, stream>>>(a, kpw);
+    if (D <= 32) rc = launch(local_shard_kernel<4, 8>, 8);
+    else rc = launch(local_shard_kernel<4, 32>, 32);
   }
+  if (rc != RS_OK) return rc;
   RS_LAUNCH_CHECK();
   return RS_OK;
 }
