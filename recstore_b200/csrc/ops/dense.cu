@@ -15,96 +15,112 @@ namespace {
 
 constexpr int kHeadMaxK = 1024;
 
-// One warp per row.  K <= 1024, K % 8 == 0.
+// One warp per row, R rows in flight.  K <= 256 * C, K % 8 == 0; lane l holds columns 8 l .. 8 l + 7 of every 256-column chunk.
+// A row is one 16-byte load per lane and chunk followed by a reduction, so a warp with one row in flight waits for memory most
+// of the time; R loads are issued together.  The weight gradient stays in registers until the block is done and leaves
+// through shared memory warp after warp: no float atomics there, which are compare-and-swap loops.
+// 65,536 x 256: 50 us with one row in flight, 3.5 waves of 64-row blocks and shared-memory atomics.
+template <int C, int R>
 __global__ void __launch_bounds__(256) head_bce_kernel(const __nv_bfloat16* __restrict__ X, int ldx, int M, int K,
                                                        const float* __restrict__ w, const float* __restrict__ bias,
                                                        const float* __restrict__ labels, float inv_batch,
                                                        float* __restrict__ prob, float* __restrict__ loss_sum,
                                                        __nv_bfloat16* __restrict__ dX, int lddx,
-                                                       float* __restrict__ dw, float* __restrict__ db,
-                                                       int rows_per_block, int with_logits_only) {
-  __shared__ float s_dw[kHeadMaxK];
-  __shared__ float s_loss, s_db;
-  for (int i = threadIdx.x; i < K; i += blockDim.x) s_dw[i] = 0.f;
-  if (threadIdx.x == 0) { s_loss = 0.f; s_db = 0.f; }
-  __syncthreads();
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nwarps = blockDim.x >> 5;
-  const int row0 = blockIdx.x * rows_per_block;
-  const int row1 = min(M, row0 + rows_per_block);
+                                                       float* __restrict__ dw, float* __restrict__ db, int with_logits_only) {
+  __shared__ float s_dw[256 * C];
+  __shared__ float s_loss[8], s_db[8];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int nvec = K >> 3;
-  const int per_lane = (nvec + 31) / 32;  // <= 4
-  float wreg[4][8];
-  float dwreg[4][8];
+  float wreg[C][8], dwreg[C][8];
 #pragma unroll
-  for (int c = 0; c < 4; ++c)
+  for (int c = 0; c < C; ++c)
 #pragma unroll
     for (int e = 0; e < 8; ++e) {
       const int v = lane + c * 32;
-      wreg[c][e] = (c < per_lane && v < nvec) ? w[v * 8 + e] : 0.f;
+      wreg[c][e] = v < nvec ? w[v * 8 + e] : 0.f;
       dwreg[c][e] = 0.f;
     }
   const float b0 = bias ? bias[0] : 0.f;
   float loss_acc = 0.f, db_acc = 0.f;
-  for (int r = row0 + warp; r < row1; r += nwarps) {
-    float xv[4][8];
-    float dot = 0.f;
+  const int nwarps = gridDim.x * 8;
+  for (long long r0 = static_cast<long long>(blockIdx.x * 8 + warp) * R; r0 < M; r0 += static_cast<long long>(nwarps) * R) {
+    uint4 raw[R][C];
+    float y[R], dot[R];
 #pragma unroll
-    for (int c = 0; c < 4; ++c) {
-      const int v = lane + c * 32;
-      if (c < per_lane && v < nvec) {
-        const uint4 raw = __ldg(reinterpret_cast<const uint4*>(X + static_cast<size_t>(r) * ldx) + v);
-        const __nv_bfloat16* xe = reinterpret_cast<const __nv_bfloat16*>(&raw);
+    for (int i = 0; i < R; ++i) {
+      const long long r = r0 + i;
+      y[i] = (!with_logits_only && r < M) ? labels[r] : 0.f;
 #pragma unroll
-        for (int e = 0; e < 8; ++e) {
-          xv[c][e] = __bfloat162float(xe[e]);
-          dot += xv[c][e] * wreg[c][e];
-        }
-      } else {
-#pragma unroll
-        for (int e = 0; e < 8; ++e) xv[c][e] = 0.f;
+      for (int c = 0; c < C; ++c) {
+        const int v = lane + c * 32;
+        raw[i][c] = (r < M && v < nvec) ? __ldg(reinterpret_cast<const uint4*>(X + r * ldx) + v) : make_uint4(0, 0, 0, 0);
       }
     }
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) dot += __shfl_xor_sync(0xffffffffu, dot, o);
-    const float z = dot + b0;
-    const float p = 1.f / (1.f + __expf(-z));
-    if (prob && lane == 0) prob[r] = p;
-    if (with_logits_only) continue;
-    const float y = labels[r];
-    // numerically stable BCE with logits: max(z,0) - z*y + log(1 + exp(-|z|))
-    const float l = fmaxf(z, 0.f) - z * y + log1pf(__expf(-fabsf(z)));
-    const float dz = (p - y) * inv_batch;
-    if (lane == 0) { loss_acc += l; db_acc += dz; }
+    for (int i = 0; i < R; ++i) {
+      dot[i] = 0.f;
 #pragma unroll
-    for (int c = 0; c < 4; ++c) {
-      const int v = lane + c * 32;
-      if (c < per_lane && v < nvec) {
+      for (int c = 0; c < C; ++c) {
+        const __nv_bfloat16* xe = reinterpret_cast<const __nv_bfloat16*>(&raw[i][c]);
+#pragma unroll
+        for (int e = 0; e < 8; ++e) dot[i] += __bfloat162float(xe[e]) * wreg[c][e];
+      }
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+      for (int i = 0; i < R; ++i) dot[i] += __shfl_xor_sync(0xffffffffu, dot[i], o);
+#pragma unroll
+    for (int i = 0; i < R; ++i) {
+      const long long r = r0 + i;
+      if (r >= M) break;
+      const float z = dot[i] + b0;
+      const float p = 1.f / (1.f + __expf(-z));
+      if (prob && lane == 0) prob[r] = p;
+      if (with_logits_only) continue;
+      // numerically stable BCE with logits: max(z,0) - z*y + log(1 + exp(-|z|))
+      const float l = fmaxf(z, 0.f) - z * y[i] + log1pf(__expf(-fabsf(z)));
+      const float dz = (p - y[i]) * inv_batch;
+      loss_acc += l;
+      db_acc += dz;
+#pragma unroll
+      for (int c = 0; c < C; ++c) {
+        const int v = lane + c * 32;
+        const __nv_bfloat16* xe = reinterpret_cast<const __nv_bfloat16*>(&raw[i][c]);
         uint4 o;
         __nv_bfloat16* oe = reinterpret_cast<__nv_bfloat16*>(&o);
 #pragma unroll
         for (int e = 0; e < 8; ++e) {
-          dwreg[c][e] += dz * xv[c][e];
-          oe[e] = __float2bfloat16(xv[c][e] > 0.f ? dz * wreg[c][e] : 0.f);
+          const float x = __bfloat162float(xe[e]);
+          dwreg[c][e] += dz * x;
+          oe[e] = __float2bfloat16(x > 0.f ? dz * wreg[c][e] : 0.f);
         }
-        if (dX) *(reinterpret_cast<uint4*>(dX + static_cast<size_t>(r) * lddx) + v) = o;
+        if (dX && v < nvec) *(reinterpret_cast<uint4*>(dX + r * lddx) + v) = o;
       }
     }
   }
   if (with_logits_only) return;
+  if (lane == 0) { s_loss[warp] = loss_acc; s_db[warp] = db_acc; }
+  for (int q = 0; q < 8; ++q) {
+    if (warp == q) {
 #pragma unroll
-  for (int c = 0; c < 4; ++c) {
-    const int v = lane + c * 32;
-    if (c < per_lane && v < nvec) {
+      for (int c = 0; c < C; ++c)
 #pragma unroll
-      for (int e = 0; e < 8; ++e) atomicAdd(&s_dw[v * 8 + e], dwreg[c][e]);
+        for (int e = 0; e < 8; ++e) {
+          const int col = (lane + c * 32) * 8 + e;
+          if (q == 0) s_dw[col] = dwreg[c][e];
+          else s_dw[col] += dwreg[c][e];
+        }
     }
+    __syncthreads();
   }
-  if (lane == 0) { atomicAdd(&s_loss, loss_acc); atomicAdd(&s_db, db_acc); }
-  __syncthreads();
   for (int i = threadIdx.x; i < K; i += blockDim.x) atomicAdd(&dw[i], s_dw[i]);
   if (threadIdx.x == 0) {
-    atomicAdd(loss_sum, s_loss * inv_batch);
-    if (db) atomicAdd(db, s_db);
+    float l = 0.f, d = 0.f;
+#pragma unroll
+    for (int q = 0; q < 8; ++q) { l += s_loss[q]; d += s_db[q]; }
+    atomicAdd(loss_sum, l * inv_batch);
+    if (db) atomicAdd(db, d);
   }
 }
 
@@ -265,6 +281,23 @@ __global__ void pad_cast_kernel(const float* __restrict__ in, int M, int K, int 
   out[i] = __float2bfloat16(k < K ? in[static_cast<size_t>(m) * ldi + k] : 0.f);
 }
 
+// Same, eight outputs per thread: one 16-byte store and one division by the row length per eight values (the one-value form
+// took 13.7 us for 65,536 x 13 -> 64, all of it index arithmetic and 2-byte stores).
+__global__ void __launch_bounds__(256) pad_cast8_kernel(const float* __restrict__ in, int M, int K, int ldi, __nv_bfloat16* __restrict__ out,
+                                                        int ldo) {
+  const unsigned per_row = static_cast<unsigned>(ldo) >> 3;
+  const unsigned i = blockIdx.x * 256u + threadIdx.x;
+  const unsigned m = i / per_row;
+  if (m >= static_cast<unsigned>(M)) return;
+  const int k0 = static_cast<int>(i - m * per_row) * 8;
+  const float* src = in + static_cast<size_t>(m) * ldi;
+  uint4 o;
+  __nv_bfloat16* oe = reinterpret_cast<__nv_bfloat16*>(&o);
+#pragma unroll
+  for (int e = 0; e < 8; ++e) oe[e] = __float2bfloat16(k0 + e < K ? src[k0 + e] : 0.f);
+  reinterpret_cast<uint4*>(out)[i] = o;
+}
+
 __global__ void mse_kernel(const __nv_bfloat16* __restrict__ pred, const float* __restrict__ target, int n,
                            float inv_n, float* __restrict__ loss_sum, __nv_bfloat16* __restrict__ dpred) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -410,10 +443,17 @@ RS_API int rs_head_bce(const void* X, int ldx, int M, int K, const float* w, con
   RS_REQUIRE(K % 8 == 0 && K <= kHeadMaxK && ldx % 8 == 0, "rs_head_bce: K=%d must be a multiple of 8, <= %d", K, kHeadMaxK);
   RS_REQUIRE(labels == nullptr || (loss_sum && dw), "rs_head_bce: training needs loss_sum and dw");
   if (M == 0) return RS_OK;
-  const int rows_per_block = 64;
-  head_bce_kernel<<<(M + rows_per_block - 1) / rows_per_block, 256, 0, stream>>>(
-      reinterpret_cast<const __nv_bfloat16*>(X), ldx, M, K, w, bias, labels, inv_batch, prob, loss_sum,
-      reinterpret_cast<__nv_bfloat16*>(dX), lddx, dw, db, rows_per_block, labels == nullptr ? 1 : 0);
+  // Rows in flight shrink with the row length (registers).  The grid gives every warp about two passes, up to what is
+  // resident at once: every block ends with K + 2 atomics on the same addresses.
+  auto launch = [&](auto kern, int R) {
+    const long long blocks = (M + 16ll * R - 1) / (16ll * R);
+    kern<<<static_cast<unsigned>(blocks < 148 * 3 ? blocks : 148 * 3), 256, 0, stream>>>(
+        reinterpret_cast<const __nv_bfloat16*>(X), ldx, M, K, w, bias, labels, inv_batch, prob, loss_sum,
+        reinterpret_cast<__nv_bfloat16*>(dX), lddx, dw, db, labels == nullptr ? 1 : 0);
+  };
+  if (K <= 256) launch(head_bce_kernel<1, 4>, 4);
+  else if (K <= 512) launch(head_bce_kernel<2, 2>, 2);
+  else launch(head_bce_kernel<4, 1>, 1);
   RS_LAUNCH_CHECK();
   return RS_OK;
 }
@@ -471,6 +511,11 @@ RS_API int rs_pad_cast_bf16(const float* in, int M, int K, int ldi, void* out, i
   RS_REQUIRE(in && out && ldo >= K, "rs_pad_cast_bf16: bad argument");
   if (M == 0) return RS_OK;
   const long long n = static_cast<long long>(M) * ldo;
+  if (ldo % 8 == 0 && (reinterpret_cast<uintptr_t>(out) & 15) == 0 && n < (1ll << 34)) {   // (32-bit thread numbers)
+    pad_cast8_kernel<<<static_cast<unsigned>((n / 8 + 255) / 256), 256, 0, stream>>>(in, M, K, ldi, reinterpret_cast<__nv_bfloat16*>(out), ldo);
+    RS_LAUNCH_CHECK();
+    return RS_OK;
+  }
   pad_cast_kernel<<<static_cast<unsigned>((n + 255) / 256), 256, 0, stream>>>(in, M, K, ldi,
                                                                                reinterpret_cast<__nv_bfloat16*>(out), ldo);
   RS_LAUNCH_CHECK();
