@@ -58,6 +58,7 @@ struct KgeArgs {
   const float* GA; const float* GB;                  // [bs, Dp], [C*ns, Dp]
   float* A32;                                        // pairwise family: a in fp32, [bs, Dp] (the GA buffer)
   float* Wf;                                         // pairwise family: d loss / d neg score, [bs, ns] (the S buffer)
+  int vec;                                           // rows can be taken in 16-byte pieces (D, Dp and all addresses allow it)
   float* pos_score; float* neg_score;                // optional outputs (evaluation / tests): [bs], [bs, ns]
 };
 
@@ -100,13 +101,50 @@ __device__ __forceinline__ void bil_bwd(int model, bool ch, float g0, float g1, 
 // distance contribution of one pair of differences and its direction (d psi / d difference)
 __device__ __forceinline__ float pair_psi(int model, float d0, float d1, float& u0, float& u1) {
   if (model == kTransE1) { u0 = sgn(d0); u1 = sgn(d1); return fabsf(d0) + fabsf(d1); }
-  const float m = sqrtf(d0 * d0 + d1 * d1);
-  const float inv = m > 0.f ? 1.f / m : 0.f;
+  const float m2 = d0 * d0 + d1 * d1;
+  const float inv = m2 > 0.f ? rsqrtf(m2) : 0.f;     // one special-function instruction where root and reciprocal take two
   u0 = d0 * inv; u1 = d1 * inv;
-  return m;
+  return m2 * inv;
 }
 __device__ __forceinline__ float pair_dist(int model, float d0, float d1) {
   return model == kTransE1 ? fabsf(d0) + fabsf(d1) : sqrtf(d0 * d0 + d1 * d1);
+}
+
+// ---- rows in 16-byte pieces (KgeArgs::vec) ---------------------------------------------------------------------------
+// A warp walks a row of a few hundred floats; loads of kRowBatch pieces per lane are issued before the first is used.  (One
+// element per lane and step, with stores between the loads, made the row kernels chains of a dozen memory latencies: prepare
+// 12.7 us and finish 17 us for 2,048 rows of 400.)
+constexpr int kRowBatch = 4;
+__device__ __forceinline__ float4 add4(const float4& a, const float4& b, float s = 1.f) {
+  return make_float4(a.x + s * b.x, a.y + s * b.y, a.z + s * b.z, a.w + s * b.w);
+}
+template <typename Load, typename Use>
+__device__ __forceinline__ void for_row4(int n, int lane, Load load, Use use) {
+  for (int d0 = lane * 4; d0 < n; d0 += 128 * kRowBatch) {
+    decltype(load(0)) v[kRowBatch];
+#pragma unroll
+    for (int u = 0; u < kRowBatch; ++u)
+      if (d0 + 128 * u < n) v[u] = load(d0 + 128 * u);
+#pragma unroll
+    for (int u = 0; u < kRowBatch; ++u)
+      if (d0 + 128 * u < n) use(d0 + 128 * u, v[u]);
+  }
+}
+// Stores four values as bf16 and returns the sum of squares of what was stored.
+__device__ __forceinline__ float store_bf16x4(__nv_bfloat16* p, const float4& v) {
+  const __nv_bfloat162 lo = __floats2bfloat162_rn(v.x, v.y), hi = __floats2bfloat162_rn(v.z, v.w);
+  uint2 o;
+  o.x = *reinterpret_cast<const uint32_t*>(&lo);
+  o.y = *reinterpret_cast<const uint32_t*>(&hi);
+  *reinterpret_cast<uint2*>(p) = o;
+  const float2 a = __bfloat1622float2(lo), b = __bfloat1622float2(hi);
+  return a.x * a.x + a.y * a.y + b.x * b.x + b.y * b.y;
+}
+__device__ __forceinline__ float4 load_bf16x4(const __nv_bfloat16* p) {
+  const uint2 o = *reinterpret_cast<const uint2*>(p);
+  const float2 a = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&o.x));
+  const float2 b = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&o.y));
+  return make_float4(a.x, a.y, b.x, b.y);
 }
 
 // one warp per row: rows [0, bs) are positives, rows [bs, bs + C*ns) negatives
@@ -118,13 +156,19 @@ __global__ void __launch_bounds__(256) kge_prepare_kernel(const KgeArgs k) {
   if (row >= k.bs) {
     if (is_pairwise(k.model)) return;                // the pairwise kernels read the fp32 rows themselves
     const int j = row - k.bs;
+    const float* src = k.neg + static_cast<size_t>(j) * D;
+    __nv_bfloat16* dst = k.Bn + static_cast<size_t>(j) * k.Dp;
     float s = 0.f;
-    for (int d = lane; d < k.Dp; d += 32) {
-      const float v = d < D ? k.neg[static_cast<size_t>(j) * D + d] : 0.f;
-      const __nv_bfloat16 b = __float2bfloat16(v);
-      k.Bn[static_cast<size_t>(j) * k.Dp + d] = b;
-      const float vb = __bfloat162float(b);
-      s += vb * vb;
+    if (k.vec) {
+      for_row4(k.Dp, lane, [&](int d) { return d < D ? *reinterpret_cast<const float4*>(src + d) : make_float4(0.f, 0.f, 0.f, 0.f); },
+               [&](int d, const float4& v) { s += store_bf16x4(dst + d, v); });
+    } else {
+      for (int d = lane; d < k.Dp; d += 32) {
+        const __nv_bfloat16 b = __float2bfloat16(d < D ? src[d] : 0.f);
+        dst[d] = b;
+        const float vb = __bfloat162float(b);
+        s += vb * vb;
+      }
     }
     s = warp_sum(s);
     if (lane == 0) k.b2[j] = s;
@@ -141,7 +185,29 @@ __global__ void __launch_bounds__(256) kge_prepare_kernel(const KgeArgs k) {
 
   if (k.model == kTransE2) {
     float a2 = 0.f, pos = 0.f;
-    for (int d = lane; d < k.Dp; d += 32) {
+    __nv_bfloat16* A = k.A + static_cast<size_t>(i) * k.Dp;
+    if (k.vec) {
+      for (int d0 = lane * 4; d0 < k.Dp; d0 += 128 * kRowBatch) {
+        float4 hv[kRowBatch], rv[kRowBatch], tv[kRowBatch];
+#pragma unroll
+        for (int u = 0; u < kRowBatch; ++u) {
+          const int d = d0 + 128 * u;
+          const float4 z = make_float4(0.f, 0.f, 0.f, 0.f);
+          hv[u] = d < D ? *reinterpret_cast<const float4*>(h + d) : z;
+          rv[u] = d < D ? *reinterpret_cast<const float4*>(r + d) : z;
+          tv[u] = d < D ? *reinterpret_cast<const float4*>(t + d) : z;
+        }
+#pragma unroll
+        for (int u = 0; u < kRowBatch; ++u) {
+          const int d = d0 + 128 * u;
+          if (d >= k.Dp) continue;
+          const float4 diff = add4(add4(hv[u], rv[u]), tv[u], -1.f);
+          a2 += store_bf16x4(A + d, k.corrupt_head ? add4(tv[u], rv[u], -1.f) : add4(hv[u], rv[u]));
+          pos += diff.x * diff.x + diff.y * diff.y + diff.z * diff.z + diff.w * diff.w;
+        }
+      }
+    }
+    for (int d = k.vec ? k.Dp : lane; d < k.Dp; d += 32) {
       float a = 0.f;
       if (d < D) {
         const float hv = h[d], rv = r[d], tv = t[d];
@@ -164,9 +230,24 @@ __global__ void __launch_bounds__(256) kge_prepare_kernel(const KgeArgs k) {
       if (k.pos_score) k.pos_score[i] = score;
       atomicAdd(&k.loss[0], -log_sigmoid(score) * inv_bs);
     }
-    for (int d = lane; d < D; d += 32) {
-      const float g = -q * (h[d] + r[d] - t[d]) / dist;   // d score / d h = -(h + r - t) / dist
-      gh[d] = g; gr[d] = g; gt[d] = -g;
+    const float qd = -q / dist;                     // d score / d h = -(h + r - t) / dist
+    if (k.vec) {
+      for_row4(D, lane,
+               [&](int d) {
+                 return add4(add4(*reinterpret_cast<const float4*>(h + d), *reinterpret_cast<const float4*>(r + d)),
+                             *reinterpret_cast<const float4*>(t + d), -1.f);
+               },
+               [&](int d, const float4& v) {
+                 const float4 g = make_float4(qd * v.x, qd * v.y, qd * v.z, qd * v.w);
+                 *reinterpret_cast<float4*>(gh + d) = g;
+                 *reinterpret_cast<float4*>(gr + d) = g;
+                 *reinterpret_cast<float4*>(gt + d) = make_float4(-g.x, -g.y, -g.z, -g.w);
+               });
+    } else {
+      for (int d = lane; d < D; d += 32) {
+        const float g = qd * (h[d] + r[d] - t[d]);
+        gh[d] = g; gr[d] = g; gt[d] = -g;
+      }
     }
     return;
   }
@@ -294,45 +375,82 @@ __global__ void __launch_bounds__(256) kge_prepare_kernel(const KgeArgs k) {
   }
 }
 
-// one thread per (positive i, negative j of its chunk); W row-major [bs, C*ns], zero outside the chunk
+// W row-major [bs, C*ns], zero outside the chunk diagonal.  A block takes 8 positives (one per warp) x 256 columns, a lane 8
+// neighbouring columns: row sums leave with one atomic per warp, column sums meet in shared memory over the 8 rows and leave
+// with one atomic per column, the loss with one per block.  (A thread per element with two global atomics each spent 37 us
+// on 524,288 atomics for 1,024 x 256 pairs; a block off the diagonal only writes zeros.)
+constexpr int kLossCols = 256;
 __global__ void __launch_bounds__(256) kge_neg_loss_kernel(const KgeArgs k) {
-  const long long idx = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x;
+  __shared__ float s_w[8][kLossCols];
+  __shared__ float s_l[8];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int ncols = k.C * k.ns;
-  float l = 0.f;
-  if (idx < static_cast<long long>(k.bs) * ncols) {
-    const int i = static_cast<int>(idx / ncols);
-    const int col = static_cast<int>(idx % ncols);
-    const int c = i / k.cs;
-    float w = 0.f;
-    if (col / k.ns == c) {
-      const float dot = k.S[idx];
+  const int i = blockIdx.y * 8 + warp;
+  const int c0 = blockIdx.x * kLossCols;
+  const int col = c0 + lane * 8;                      // (ncols is a multiple of 8: the GEMM asks for it)
+  const bool row_ok = i < k.bs;
+  const int c = row_ok ? i / k.cs : 0;
+  const int lo = c * k.ns, hi = lo + k.ns;            // the columns of this row's chunk
+  float w[8], l = 0.f, rs = 0.f;
+#pragma unroll
+  for (int e = 0; e < 8; ++e) w[e] = 0.f;
+  if (row_ok && col < hi && col + 8 > lo && col < ncols) {
+    const float* sp = k.S + static_cast<size_t>(i) * ncols + col;
+    const float4 s0 = *reinterpret_cast<const float4*>(sp), s1 = *reinterpret_cast<const float4*>(sp + 4);
+    const float dot[8] = {s0.x, s0.y, s0.z, s0.w, s1.x, s1.y, s1.z, s1.w};
+    const float norm = 1.f / (static_cast<float>(k.bs) * k.ns) * 0.5f;
+    const float a2 = k.model == kTransE2 ? k.a2[i] : 0.f;
+#pragma unroll
+    for (int e = 0; e < 8; ++e) {
+      if (col + e < lo || col + e >= hi) continue;
       float score, wgt;
-      const float norm = 1.f / (static_cast<float>(k.bs) * k.ns) * 0.5f;
       if (k.model == kTransE2) {
-        const float dist = sqrtf(fmaxf(k.a2[i] + k.b2[col] - 2.f * dot, 1e-30f));
+        const float dist = sqrtf(fmaxf(a2 + k.b2[col + e] - 2.f * dot[e], 1e-30f));
         score = k.gamma - dist;
         wgt = sigmoid(score) * norm / dist;      // q / dist
       } else if (k.model == kSimplE) {
-        score = fminf(fmaxf(dot, -20.f), 20.f);
-        wgt = (dot >= -20.f && dot <= 20.f) ? sigmoid(score) * norm : 0.f;
+        score = fminf(fmaxf(dot[e], -20.f), 20.f);
+        wgt = (dot[e] >= -20.f && dot[e] <= 20.f) ? sigmoid(score) * norm : 0.f;
       } else {
-        score = dot;
+        score = dot[e];
         wgt = sigmoid(score) * norm;             // q
       }
-      l = -log_sigmoid(-score) * norm;
-      w = wgt;
-      if (k.neg_score) k.neg_score[static_cast<size_t>(i) * k.ns + (col - c * k.ns)] = score;
-      const __nv_bfloat16 wb = __float2bfloat16(w);
-      w = __bfloat162float(wb);
-      atomicAdd(&k.rowsum[i], w);
-      atomicAdd(&k.colsum[col], w);
-      k.W[idx] = wb;
-    } else {
-      k.W[idx] = __float2bfloat16(0.f);
+      l -= log_sigmoid(-score) * norm;
+      if (k.neg_score) k.neg_score[static_cast<size_t>(i) * k.ns + (col + e - lo)] = score;
+      w[e] = __bfloat162float(__float2bfloat16(wgt));
+      rs += w[e];
     }
   }
+  if (row_ok && col < ncols) {
+    uint4 o;
+    __nv_bfloat16* oe = reinterpret_cast<__nv_bfloat16*>(&o);
+#pragma unroll
+    for (int e = 0; e < 8; ++e) oe[e] = __float2bfloat16(w[e]);
+    *reinterpret_cast<uint4*>(k.W + static_cast<size_t>(i) * ncols + col) = o;
+  }
+  // off the diagonal for all of the block's rows: zeros are written, nothing is left to add
+  const int first = blockIdx.y * 8, last = min(k.bs, first + 8) - 1;
+  if (c0 >= (last / k.cs + 1) * k.ns || c0 + kLossCols <= (first / k.cs) * k.ns) return;
+  rs = warp_sum(rs);
   l = warp_sum(l);
-  if ((threadIdx.x & 31) == 0 && l != 0.f) atomicAdd(&k.loss[1], l);
+  if (lane == 0) {
+    if (row_ok && rs != 0.f) atomicAdd(&k.rowsum[i], rs);
+    s_l[warp] = l;
+  }
+  *reinterpret_cast<float4*>(&s_w[warp][lane * 8]) = make_float4(w[0], w[1], w[2], w[3]);
+  *reinterpret_cast<float4*>(&s_w[warp][lane * 8 + 4]) = make_float4(w[4], w[5], w[6], w[7]);
+  __syncthreads();
+  const int my = c0 + threadIdx.x;
+  float cs = 0.f;
+#pragma unroll
+  for (int q = 0; q < 8; ++q) cs += s_w[q][threadIdx.x];
+  if (my < ncols && cs != 0.f) atomicAdd(&k.colsum[my], cs);
+  if (threadIdx.x == 0) {
+    float t = 0.f;
+#pragma unroll
+    for (int q = 0; q < 8; ++q) t += s_l[q];
+    if (t != 0.f) atomicAdd(&k.loss[1], t);
+  }
 }
 
 // one warp per row again
@@ -343,7 +461,20 @@ __global__ void __launch_bounds__(256) kge_finish_kernel(const KgeArgs k) {
   if (row >= k.bs + k.C * k.ns) return;
   if (row >= k.bs) {
     const int j = row - k.bs;
-    const float cs = k.colsum[j];
+    const float cs = k.model == kTransE2 ? k.colsum[j] : 0.f;
+    if (k.vec) {
+      const float* gb = k.GB + static_cast<size_t>(j) * k.Dp;
+      const __nv_bfloat16* bn = k.Bn + static_cast<size_t>(j) * k.Dp;
+      float* out = k.gneg + static_cast<size_t>(j) * D;
+      const bool centred = k.model == kTransE2;
+      for_row4(D, lane,
+               [&](int d) {
+                 const float4 g = *reinterpret_cast<const float4*>(gb + d);
+                 return centred ? add4(g, load_bf16x4(bn + d), -cs) : g;
+               },
+               [&](int d, const float4& g) { *reinterpret_cast<float4*>(out + d) = g; });
+      return;
+    }
     for (int d = lane; d < D; d += 32) {
       float g = k.GB[static_cast<size_t>(j) * k.Dp + d];
       if (k.model == kTransE2) g -= cs * __bfloat162float(k.Bn[static_cast<size_t>(j) * k.Dp + d]);
@@ -358,6 +489,30 @@ __global__ void __launch_bounds__(256) kge_finish_kernel(const KgeArgs k) {
   const float* GA = k.GA + static_cast<size_t>(i) * k.Dp;
   if (k.model == kTransE2) {
     const float rs = k.rowsum[i];
+    if (k.vec) {
+      const __nv_bfloat16* A = k.A + static_cast<size_t>(i) * k.Dp;
+      float* gx = k.corrupt_head ? gt : gh;                   // a = t - r  or  a = h + r
+      const float sr = k.corrupt_head ? -1.f : 1.f;
+      for (int d0 = lane * 4; d0 < D; d0 += 128 * kRowBatch) {
+        float4 ga[kRowBatch], x[kRowBatch], r[kRowBatch];
+#pragma unroll
+        for (int u = 0; u < kRowBatch; ++u) {
+          const int d = d0 + 128 * u;
+          if (d >= D) continue;
+          ga[u] = add4(*reinterpret_cast<const float4*>(GA + d), load_bf16x4(A + d), -rs);
+          x[u] = *reinterpret_cast<const float4*>(gx + d);
+          r[u] = *reinterpret_cast<const float4*>(gr + d);
+        }
+#pragma unroll
+        for (int u = 0; u < kRowBatch; ++u) {
+          const int d = d0 + 128 * u;
+          if (d >= D) continue;
+          *reinterpret_cast<float4*>(gx + d) = add4(x[u], ga[u]);
+          *reinterpret_cast<float4*>(gr + d) = add4(r[u], ga[u], sr);
+        }
+      }
+      return;
+    }
     for (int d = lane; d < D; d += 32) {
       const float ga = GA[d] - rs * __bfloat162float(k.A[static_cast<size_t>(i) * k.Dp + d]);
       if (k.corrupt_head) { gt[d] += ga; gr[d] -= ga; }    // a = t - r
@@ -442,36 +597,40 @@ __global__ void __launch_bounds__(256) kge_finish_kernel(const KgeArgs k) {
 }
 
 // ---- pairwise family ---------------------------------------------------------------------------------------------
-// A warp scores 4 positives against 8 negatives of their chunk: every lane strides over the element pairs and keeps
-// 32 partial distances, which a transposing butterfly reduces so that lane l ends with pair (l / 8, l % 8).
-__global__ void __launch_bounds__(256) kge_pair_forward_kernel(const KgeArgs k) {
+// A warp scores 4 positives against 4 negatives of their chunk: every lane strides over the element pairs and keeps
+// 16 partial distances, which a transposing butterfly reduces so that lanes 2 p and 2 p + 1 end with pair p = (p / 4, p % 4).
+// Bound by latency and issue slots, operands come from L1 / L2: 16 sums leave room for twice the warps that 4 x 8 pairs did
+// (114 registers, 23 % of the warps resident, 53 us for 1,024 x 256 pairs of 200 complex elements).
+constexpr int kPairTileI = 4, kPairTileJ = 4;
+template <int MODEL>
+__global__ void __launch_bounds__(256, 4) kge_pair_forward_kernel(const KgeArgs k) {
   const int lane = threadIdx.x & 31;
   const int warp = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-  const int jt = k.ns >> 3;                        // tiles of 8 negatives per chunk
-  const int n_warps = (k.bs >> 2) * jt;
+  const int jt = k.ns / kPairTileJ;                // tiles of negatives per chunk
+  const int n_warps = (k.bs / kPairTileI) * jt;
   float l = 0.f;
   if (warp < n_warps) {
-    const int i0 = (warp / jt) << 2, j0 = (warp % jt) << 3;
+    const int i0 = (warp / jt) * kPairTileI, j0 = (warp % jt) * kPairTileJ;
     const int c = i0 / k.cs;
     const int H = k.D >> 1;
     const float* a = k.A32 + static_cast<size_t>(i0) * k.Dp;
     const float* n = k.neg + (static_cast<size_t>(c) * k.ns + j0) * k.D;
-    float v[32];
+    float v[16];
 #pragma unroll
-    for (int p = 0; p < 32; ++p) v[p] = 0.f;
+    for (int p = 0; p < 16; ++p) v[p] = 0.f;
     for (int kk = lane; kk < H; kk += 32) {
-      float a0[4], a1[4], n0[8], n1[8];
+      float a0[4], a1[4], n0[4], n1[4];
 #pragma unroll
       for (int ii = 0; ii < 4; ++ii) { a0[ii] = a[ii * k.Dp + kk]; a1[ii] = a[ii * k.Dp + kk + H]; }
 #pragma unroll
-      for (int jj = 0; jj < 8; ++jj) { n0[jj] = n[jj * k.D + kk]; n1[jj] = n[jj * k.D + kk + H]; }
+      for (int jj = 0; jj < 4; ++jj) { n0[jj] = n[jj * k.D + kk]; n1[jj] = n[jj * k.D + kk + H]; }
 #pragma unroll
       for (int ii = 0; ii < 4; ++ii)
 #pragma unroll
-        for (int jj = 0; jj < 8; ++jj) v[ii * 8 + jj] += pair_dist(k.model, a0[ii] - n0[jj], a1[ii] - n1[jj]);
+        for (int jj = 0; jj < 4; ++jj) v[ii * 4 + jj] += pair_dist(MODEL, a0[ii] - n0[jj], a1[ii] - n1[jj]);
     }
 #pragma unroll
-    for (int o = 16, cnt = 32; o > 0; o >>= 1, cnt >>= 1) {
+    for (int o = 16, cnt = 16; o > 1; o >>= 1, cnt >>= 1) {
       const bool upper = (lane & o) != 0;
 #pragma unroll
       for (int p = 0; p < cnt / 2; ++p) {
@@ -480,12 +639,16 @@ __global__ void __launch_bounds__(256) kge_pair_forward_kernel(const KgeArgs k) 
         v[p] = keep + __shfl_xor_sync(0xffffffffu, send, o);
       }
     }
-    const int i = i0 + (lane >> 3), j = j0 + (lane & 7);
-    const float score = k.gamma - v[0];
-    const float norm = 1.f / (static_cast<float>(k.bs) * k.ns) * 0.5f;
-    k.Wf[static_cast<size_t>(i) * k.ns + j] = sigmoid(score) * norm;     // d loss / d score
-    if (k.neg_score) k.neg_score[static_cast<size_t>(i) * k.ns + j] = score;
-    l = -log_sigmoid(-score) * norm;
+    v[0] += __shfl_xor_sync(0xffffffffu, v[0], 1);
+    if ((lane & 1) == 0) {
+      const int p = lane >> 1;
+      const int i = i0 + (p >> 2), j = j0 + (p & 3);
+      const float score = k.gamma - v[0];
+      const float norm = 1.f / (static_cast<float>(k.bs) * k.ns) * 0.5f;
+      k.Wf[static_cast<size_t>(i) * k.ns + j] = sigmoid(score) * norm;     // d loss / d score
+      if (k.neg_score) k.neg_score[static_cast<size_t>(i) * k.ns + j] = score;
+      l = -log_sigmoid(-score) * norm;
+    }
   }
   l = warp_sum(l);
   if (lane == 0 && l != 0.f) atomicAdd(&k.loss[1], l);
@@ -493,16 +656,47 @@ __global__ void __launch_bounds__(256) kge_pair_forward_kernel(const KgeArgs k) 
 
 constexpr int kPairRows = 8;      // rows that share one pass over the other side
 constexpr int kPairTile = 256;    // weights staged per pass
-constexpr int kPairThreads = 128;
+constexpr int kPairCols = 64;     // element pairs per block
+constexpr int kPairWays = 4;      // threads that share an element pair, each walking its part of the other side
+constexpr int kPairThreads = kPairCols * kPairWays;
+constexpr int kPairBatch = 4;     // rows of the other side a thread fetches at once
 
-// Block = 8 positives of one chunk x a slab of 128 element pairs; a thread owns one pair index of all 8 rows, walks
-// the chunk's negatives and then chains d loss / d a (negatives and the positive) to x and r.
+// Sums the kPairWays partial gradients of every element pair into the threads of way 0.
+__device__ __forceinline__ void pair_join(float (&g0)[kPairRows], float (&g1)[kPairRows], float* buf, int col, int way) {
+  for (int q = 1; q < kPairWays; ++q) {
+    __syncthreads();
+    if (way == q) {
+#pragma unroll
+      for (int rr = 0; rr < kPairRows; ++rr) {
+        buf[(2 * rr) * kPairCols + col] = g0[rr];
+        buf[(2 * rr + 1) * kPairCols + col] = g1[rr];
+      }
+    }
+    __syncthreads();
+    if (way == 0) {
+#pragma unroll
+      for (int rr = 0; rr < kPairRows; ++rr) {
+        g0[rr] += buf[(2 * rr) * kPairCols + col];
+        g1[rr] += buf[(2 * rr + 1) * kPairCols + col];
+      }
+    }
+  }
+}
+
+// The two gradient kernels: a block owns 8 rows of one side x 64 element pairs; its 4 ways of threads walk a quarter of the
+// other side's rows of the chunk each and add up at the end, so every gradient element still has one owner and no atomics.
+// Bound by issue slots (about a dozen instructions and one special function per element of a pair); one way of 128 threads
+// left three quarters of the warps out: 167 and 159 us for 1,024 x 256 pairs of 200 complex elements, 9 % resident.
+
+// Block = 8 positives of one chunk; chains d loss / d a (negatives and the positive) to x and r.
+template <int MODEL>
 __global__ void __launch_bounds__(kPairThreads) kge_pair_grad_pos_kernel(const KgeArgs k) {
-  __shared__ float w[kPairRows][kPairTile];
+  __shared__ __align__(16) float w[kPairTile][kPairRows];      // (the join's 16 x 64 floats fit into it)
   const int i0 = blockIdx.x * kPairRows;
   const int c = i0 / k.cs;
   const int H = k.D >> 1;
-  const int kk = blockIdx.y * kPairThreads + threadIdx.x;
+  const int col = threadIdx.x % kPairCols, way = threadIdx.x / kPairCols;
+  const int kk = blockIdx.y * kPairCols + col;
   const bool live = kk < H;
   float a0[kPairRows], a1[kPairRows], g0[kPairRows], g1[kPairRows];
 #pragma unroll
@@ -516,23 +710,37 @@ __global__ void __launch_bounds__(kPairThreads) kge_pair_grad_pos_kernel(const K
     __syncthreads();
     for (int e = threadIdx.x; e < kPairRows * nj; e += kPairThreads) {
       const int rr = e / nj, j = e - rr * nj;
-      w[rr][j] = k.Wf[static_cast<size_t>(i0 + rr) * k.ns + jb + j];
+      w[j][rr] = k.Wf[static_cast<size_t>(i0 + rr) * k.ns + jb + j];
     }
     __syncthreads();
     if (live) {
       const float* n = k.neg + (static_cast<size_t>(c) * k.ns + jb) * k.D + kk;
-      for (int j = 0; j < nj; ++j) {
-        const float n0 = n[static_cast<size_t>(j) * k.D], n1 = n[static_cast<size_t>(j) * k.D + H];
+      // kPairBatch rows of the other side are fetched together
+      for (int jj0 = way; jj0 < nj; jj0 += kPairWays * kPairBatch) {
+        float n0[kPairBatch], n1[kPairBatch];
 #pragma unroll
-        for (int rr = 0; rr < kPairRows; ++rr) {
-          float u0, u1;
-          pair_psi(k.model, a0[rr] - n0, a1[rr] - n1, u0, u1);
-          g0[rr] -= w[rr][j] * u0; g1[rr] -= w[rr][j] * u1;
+        for (int q = 0; q < kPairBatch; ++q) {
+          const float* p = n + static_cast<size_t>(min(jj0 + q * kPairWays, nj - 1)) * k.D;
+          n0[q] = p[0]; n1[q] = p[H];
+        }
+#pragma unroll
+        for (int q = 0; q < kPairBatch; ++q) {
+          const int j = jj0 + q * kPairWays;
+          if (j >= nj) break;
+          const float4 wa = *reinterpret_cast<const float4*>(&w[j][0]), wb = *reinterpret_cast<const float4*>(&w[j][4]);
+          const float ww[kPairRows] = {wa.x, wa.y, wa.z, wa.w, wb.x, wb.y, wb.z, wb.w};
+#pragma unroll
+          for (int rr = 0; rr < kPairRows; ++rr) {
+            float u0, u1;
+            pair_psi(MODEL, a0[rr] - n0[q], a1[rr] - n1[q], u0, u1);
+            g0[rr] -= ww[rr] * u0; g1[rr] -= ww[rr] * u1;
+          }
         }
       }
     }
   }
-  if (!live) return;
+  pair_join(g0, g1, &w[0][0], col, way);
+  if (!live || way != 0) return;
   const bool ch = k.corrupt_head != 0;
   const float sg = ch ? -1.f : 1.f;
   const float to_phase = kPi / k.emb_init;
@@ -544,10 +752,10 @@ __global__ void __launch_bounds__(kPairThreads) kge_pair_grad_pos_kernel(const K
     float* gx = (ch ? k.gt : k.gh) + static_cast<size_t>(i) * k.D;
     float* gr = k.gr + static_cast<size_t>(i) * k.Dr;
     float u0, u1;
-    pair_psi(k.model, a0[rr] - y[kk], a1[rr] - y[kk + H], u0, u1);
+    pair_psi(MODEL, a0[rr] - y[kk], a1[rr] - y[kk + H], u0, u1);
     const float q = k.a2[i];
     const float ga0 = g0[rr] - q * u0, ga1 = g1[rr] - q * u1;
-    if (k.model == kTransE1) {
+    if (MODEL == kTransE1) {
       gx[kk] = ga0; gx[kk + H] = ga1; gr[kk] = sg * ga0; gr[kk + H] = sg * ga1;
     } else {
       float sn, cs_;
@@ -561,13 +769,15 @@ __global__ void __launch_bounds__(kPairThreads) kge_pair_grad_pos_kernel(const K
   }
 }
 
-// Block = 8 negatives of one chunk x a slab of 128 element pairs; a thread walks the chunk's positives.
+// Block = 8 negatives of one chunk; its threads walk the chunk's positives.
+template <int MODEL>
 __global__ void __launch_bounds__(kPairThreads) kge_pair_grad_neg_kernel(const KgeArgs k) {
-  __shared__ float w[kPairTile][kPairRows];
+  __shared__ __align__(16) float w[kPairTile][kPairRows];
   const int col0 = blockIdx.x * kPairRows;          // index into [C*ns]
   const int c = col0 / k.ns, j0 = col0 - c * k.ns;
   const int H = k.D >> 1;
-  const int kk = blockIdx.y * kPairThreads + threadIdx.x;
+  const int col = threadIdx.x % kPairCols, way = threadIdx.x / kPairCols;
+  const int kk = blockIdx.y * kPairCols + col;
   const bool live = kk < H;
   float n0[kPairRows], n1[kPairRows], g0[kPairRows], g1[kPairRows];
 #pragma unroll
@@ -586,18 +796,31 @@ __global__ void __launch_bounds__(kPairThreads) kge_pair_grad_neg_kernel(const K
     __syncthreads();
     if (live) {
       const float* a = k.A32 + static_cast<size_t>(c * k.cs + ib) * k.Dp + kk;
-      for (int ii = 0; ii < ni; ++ii) {
-        const float a0 = a[static_cast<size_t>(ii) * k.Dp], a1 = a[static_cast<size_t>(ii) * k.Dp + H];
+      for (int ii0 = way; ii0 < ni; ii0 += kPairWays * kPairBatch) {
+        float a0[kPairBatch], a1[kPairBatch];
 #pragma unroll
-        for (int jj = 0; jj < kPairRows; ++jj) {
-          float u0, u1;
-          pair_psi(k.model, a0 - n0[jj], a1 - n1[jj], u0, u1);
-          g0[jj] += w[ii][jj] * u0; g1[jj] += w[ii][jj] * u1;     // d loss / d dist = -w, d dist / d e' = -u
+        for (int q = 0; q < kPairBatch; ++q) {
+          const float* p = a + static_cast<size_t>(min(ii0 + q * kPairWays, ni - 1)) * k.Dp;
+          a0[q] = p[0]; a1[q] = p[H];
+        }
+#pragma unroll
+        for (int q = 0; q < kPairBatch; ++q) {
+          const int ii = ii0 + q * kPairWays;
+          if (ii >= ni) break;
+          const float4 wa = *reinterpret_cast<const float4*>(&w[ii][0]), wb = *reinterpret_cast<const float4*>(&w[ii][4]);
+          const float ww[kPairRows] = {wa.x, wa.y, wa.z, wa.w, wb.x, wb.y, wb.z, wb.w};
+#pragma unroll
+          for (int jj = 0; jj < kPairRows; ++jj) {
+            float u0, u1;
+            pair_psi(MODEL, a0[q] - n0[jj], a1[q] - n1[jj], u0, u1);
+            g0[jj] += ww[jj] * u0; g1[jj] += ww[jj] * u1;     // d loss / d dist = -w, d dist / d e' = -u
+          }
         }
       }
     }
   }
-  if (!live) return;
+  pair_join(g0, g1, &w[0][0], col, way);
+  if (!live || way != 0) return;
 #pragma unroll
   for (int jj = 0; jj < kPairRows; ++jj) {
     k.gneg[static_cast<size_t>(col0 + jj) * k.D + kk] = g0[jj];
@@ -631,25 +854,32 @@ RS_API int rs_kge_stage(int stage, const float* h, const float* r, const float* 
   k.gh = gh; k.gr = gr; k.gt = gt; k.gneg = gneg; k.S = S; k.W = reinterpret_cast<__nv_bfloat16*>(W);
   k.rowsum = rowsum; k.colsum = colsum; k.GA = GA; k.GB = GB; k.A32 = GA; k.Wf = S;
   k.pos_score = pos_score; k.neg_score = neg_score;
+  uintptr_t bits = 0;
+  const void* const rows16[] = {h, r, t, neg, gh, gr, gt, gneg, GA, GB, A, Bn};
+  for (const void* q : rows16) bits |= reinterpret_cast<uintptr_t>(q);
+  k.vec = D % 4 == 0 && Dp % 8 == 0 && (bits & 15) == 0;
   const int rows = bs + k.C * ns;
   const int H = D / 2;
   if (stage == 0) {
     kge_prepare_kernel<<<((pairwise ? bs : rows) + 7) / 8, 256, 0, stream>>>(k);
   } else if (stage == 1) {
     if (pairwise) {
-      const int warps = (bs / 4) * (ns / 8);
-      kge_pair_forward_kernel<<<(warps + 7) / 8, 256, 0, stream>>>(k);
+      const int warps = (bs / kPairTileI) * (ns / kPairTileJ);
+      if (model == kTransE1) kge_pair_forward_kernel<kTransE1><<<(warps + 7) / 8, 256, 0, stream>>>(k);
+      else kge_pair_forward_kernel<kRotatE><<<(warps + 7) / 8, 256, 0, stream>>>(k);
     } else {
-      const long long n = static_cast<long long>(bs) * k.C * ns;
-      kge_neg_loss_kernel<<<static_cast<unsigned>((n + 255) / 256), 256, 0, stream>>>(k);
+      RS_REQUIRE((k.C * ns) % 8 == 0, "rs_kge_stage: the number of negatives (%d) must be a multiple of 8", k.C * ns);
+      kge_neg_loss_kernel<<<dim3((k.C * ns + kLossCols - 1) / kLossCols, (bs + 7) / 8), 256, 0, stream>>>(k);
     }
   } else if (stage == 2) {
     if (pairwise) {
-      const dim3 gp(bs / kPairRows, (H + kPairThreads - 1) / kPairThreads);
-      kge_pair_grad_pos_kernel<<<gp, kPairThreads, 0, stream>>>(k);
+      const dim3 gp(bs / kPairRows, (H + kPairCols - 1) / kPairCols);
+      if (model == kTransE1) kge_pair_grad_pos_kernel<kTransE1><<<gp, kPairThreads, 0, stream>>>(k);
+      else kge_pair_grad_pos_kernel<kRotatE><<<gp, kPairThreads, 0, stream>>>(k);
       RS_LAUNCH_CHECK();
-      const dim3 gn(k.C * ns / kPairRows, (H + kPairThreads - 1) / kPairThreads);
-      kge_pair_grad_neg_kernel<<<gn, kPairThreads, 0, stream>>>(k);
+      const dim3 gn(k.C * ns / kPairRows, (H + kPairCols - 1) / kPairCols);
+      if (model == kTransE1) kge_pair_grad_neg_kernel<kTransE1><<<gn, kPairThreads, 0, stream>>>(k);
+      else kge_pair_grad_neg_kernel<kRotatE><<<gn, kPairThreads, 0, stream>>>(k);
     } else {
       kge_finish_kernel<<<(rows + 7) / 8, 256, 0, stream>>>(k);
     }

@@ -130,11 +130,11 @@ class KGEModel:
         self.b2 = torch.empty(self.nneg, **f)
         self.S = torch.empty(self.bs, self.nneg, **f)
         self.W = torch.empty(self.bs, self.nneg, **b)
-        self.rowsum = torch.empty(self.bs, **f)
-        self.colsum = torch.empty(self.nneg, **f)
+        # accumulators of a step, side by side so that one fill clears them: loss [2] (+ 2 unused), row sums, column sums
+        self._sums = torch.zeros(4 + self.bs + self.nneg, **f)
+        self.loss, self.rowsum, self.colsum = self._sums[:2], self._sums[4:4 + self.bs], self._sums[4 + self.bs:]
         self.GA = torch.empty(self.bs, self.Dp, **f)
         self.GB = torch.empty(self.nneg, self.Dp, **f)
-        self.loss = torch.zeros(2, **f)
         self.pos_score = torch.empty(self.bs, **f)
         self.neg_score = torch.empty(self.bs, self.ns, **f)
         self.ids = torch.empty(n_ids, dtype=torch.int64, device=dev)
@@ -143,8 +143,9 @@ class KGEModel:
         self.heartbeat_timeout_s = 2.0
         self.launches_per_step = 0
         self._graphs: Dict[bool, torch.cuda.CUDAGraph] = {}
-        self._g_ids = (torch.zeros(self.bs, dtype=torch.int64, device=dev), torch.zeros(self.bs, dtype=torch.int64, device=dev),
-                       torch.zeros(self.bs, dtype=torch.int64, device=dev), torch.zeros(self.nneg, dtype=torch.int64, device=dev))
+        # fixed id buffers of the captured step: the entity ids where the lookup reads them
+        bs = self.bs
+        self._g_ids = (self.ids[:bs], torch.zeros(bs, dtype=torch.int64, device=dev), self.ids[bs:2 * bs], self.ids[2 * bs:])
         self._g_loss = torch.zeros((), **f)
         self._cap_stream: Optional[torch.cuda.Stream] = None
 
@@ -161,7 +162,7 @@ class KGEModel:
 
     def _forward(self, corrupt_head: bool, want_scores: bool):
         st = self.ctx.status
-        self.loss.zero_(); self.rowsum.zero_(); self.colsum.zero_()
+        self._sums.zero_()
         self._stage(0, corrupt_head, want_scores)
         if not self.pairwise:
             F_.gemm_bf16(self.A, self.Bn, self.S, mode=0, epi=F_.EPI_F32, status=st)
@@ -169,7 +170,8 @@ class KGEModel:
 
     def _fetch(self, h_ids, r_ids, t_ids, neg_ids):
         bs = self.bs
-        self.ids[:bs].copy_(h_ids); self.ids[bs:2 * bs].copy_(t_ids); self.ids[2 * bs:].copy_(neg_ids)
+        if h_ids is not self._g_ids[0]:
+            self.ids[:bs].copy_(h_ids); self.ids[bs:2 * bs].copy_(t_ids); self.ids[2 * bs:].copy_(neg_ids)
         self.entity.lookup(self.ids, out=self.ent_rows)
         if self.rescal:
             self._rel_keys.copy_((r_ids.view(-1, 1) * self.D + self._row_of_block).view(-1))
@@ -267,7 +269,7 @@ class KGEModel:
             self.relation.update(self.rel_grad.view(self.bs * self.D, self.D), norms=self._rel_norm)
         else:
             self.relation.update(self.rel_grad)
-        self.launches_per_step = (7 if self.pairwise else 9) + self.entity.launches + self.relation.launches
+        self.launches_per_step = (5 if self.pairwise else 7) + self.entity.launches + self.relation.launches
         return self.loss.sum()
 
     @torch.no_grad()
