@@ -44,12 +44,6 @@ __device__ __forceinline__ void copy_row(float* __restrict__ dst, const float* _
   for (int v = lane; v < (dim >> 2); v += 32) reinterpret_cast<float4*>(dst)[v] = reinterpret_cast<const float4*>(src)[v];
 }
 
-// Same copy with the source read from L2 (never from a possibly stale L1 line): used by the lock-free hit path, whose
-// sequence-number check only vouches for what L2 holds.
-__device__ __forceinline__ void copy_row_cg(float* __restrict__ dst, const float* src, int dim, int lane) {
-  for (int v = lane; v < (dim >> 2); v += 32) reinterpret_cast<float4*>(dst)[v] = __ldcg(reinterpret_cast<const float4*>(src) + v);
-}
-
 __global__ void cache_init_kernel(CacheView c) {
   const unsigned long long i = static_cast<unsigned long long>(blockIdx.x) * blockDim.x + threadIdx.x;
   if (i < c.nsets * kWays) {
@@ -67,79 +61,106 @@ __global__ void cache_tick_kernel(unsigned* clock, int* miss_count) {
   if (miss_count) *miss_count = 0;
 }
 
-// One warp per key: the 32 lanes compare the 32 tags of the key's set (one 256-B line).  A warp takes its keys four at a
-// time so that four tag lines are in flight before the first is compared, and it collects its misses in registers
-// (lane r keeps the r-th miss) and appends them with ONE atomicAdd per 32 misses: a counter bumped once per missing key
-// serialises the whole grid on one L2 address when the hit rate is low.
+// Eight lanes per key: each compares four of the 32 tags of the key's set (one 32-byte load), so a warp probes four keys per
+// step and keeps four steps (16 keys) in flight; the set of a key, a 64-bit remainder, is worked out by one lane and not by
+// all that probe it.  Hits are validated like a seqlock reader (version, key, row, version again), in three phases over the
+// 16 keys, so that the warp pays three dependent round trips and two fences per 16 keys.  Misses are gathered over the warp
+// and appended with one atomicAdd: a counter bumped once per missing key serialises the whole grid on one L2 address when the
+// hit rate is low.  Bound by latency; a warp per key, four keys in flight, took 45 us for 65,536 keys x 32 floats at 70 % hits.
+constexpr int kProbeLanes = 8;
+constexpr int kProbeSteps = 4;
+constexpr int kProbeKeys = 32 / kProbeLanes * kProbeSteps;    // keys per warp and pass
+
+__device__ __forceinline__ void load_tags(unsigned long long (&t)[4], const unsigned long long* p) {
+  asm volatile("ld.global.cg.v4.u64 {%0,%1,%2,%3}, [%4];" : "=l"(t[0]), "=l"(t[1]), "=l"(t[2]), "=l"(t[3]) : "l"(p) : "memory");
+}
+// Index of `key` among the four tags of this lane, or -1.
+__device__ __forceinline__ int match_tags(const unsigned long long (&t)[4], unsigned long long key) {
+  return t[0] == key ? 0 : t[1] == key ? 1 : t[2] == key ? 2 : t[3] == key ? 3 : -1;
+}
+
 __global__ void __launch_bounds__(256) cache_query_kernel(CacheView c, const long long* __restrict__ keys, long long n,
                                                           float* __restrict__ out, long long* __restrict__ miss_index,
                                                           long long* __restrict__ miss_keys, int* __restrict__ miss_count) {
-  constexpr int kAhead = 4;
-  const int lane = threadIdx.x & 31;
-  const long long warp = static_cast<long long>(blockIdx.x) * (blockDim.x >> 5) + (threadIdx.x >> 5);
+  constexpr unsigned kAll = 0xffffffffu;
+  const int lane = threadIdx.x & 31, l = lane & (kProbeLanes - 1), sub = lane / kProbeLanes;
   const long long nwarps = static_cast<long long>(gridDim.x) * (blockDim.x >> 5);
   const unsigned now = *c.clock;
-  int n_miss = 0;
-  long long my_miss_index = 0;
-  unsigned long long my_miss_key = 0;
-  auto flush_misses = [&]() {
-    int base = 0;
-    if (lane == 0) base = atomicAdd(miss_count, n_miss);
-    base = __shfl_sync(0xffffffffu, base, 0);
-    if (lane < n_miss) {
-      miss_index[base + lane] = my_miss_index;
-      miss_keys[base + lane] = static_cast<long long>(my_miss_key);
+  for (long long i0 = (static_cast<long long>(blockIdx.x) * (blockDim.x >> 5) + (threadIdx.x >> 5)) * kProbeKeys; i0 < n;
+       i0 += nwarps * kProbeKeys) {
+    unsigned long long my_key = kEmptyKey, my_set = 0;
+    if (lane < kProbeKeys && i0 + lane < n) {
+      my_key = static_cast<unsigned long long>(keys[i0 + lane]);
+      my_set = ht_hash(my_key) % c.nsets;
     }
-    n_miss = 0;
-  };
-  for (long long i0 = warp; i0 < n; i0 += nwarps * kAhead) {
-    unsigned long long key[kAhead], set[kAhead], line[kAhead];
+    unsigned long long key[kProbeSteps], slot[kProbeSteps], tags[kProbeSteps][4];
 #pragma unroll
-    for (int u = 0; u < kAhead; ++u) {
-      const long long i = i0 + u * nwarps;
-      key[u] = i < n ? static_cast<unsigned long long>(keys[i]) : kEmptyKey;
-      set[u] = ht_hash(key[u]) % c.nsets;
-      line[u] = key[u] != kEmptyKey ? c.keys[set[u] * kWays + lane] : kEmptyKey;
+    for (int u = 0; u < kProbeSteps; ++u) {
+      const int j = u * (32 / kProbeLanes) + sub;
+      key[u] = __shfl_sync(kAll, my_key, j);
+      slot[u] = __shfl_sync(kAll, my_set, j) * kWays;        // first slot of the set, for now
+      if (key[u] != kEmptyKey) load_tags(tags[u], c.keys + slot[u] + l * 4);
     }
-    // Hits are validated like a seqlock reader (version, key, row, version again), in three phases over the four keys so
-    // that the warp pays three dependent round trips and two fences per FOUR keys, not per key.
-    unsigned long long slot[kAhead], k0[kAhead];
-    unsigned v0[kAhead];
-    bool hit[kAhead];
+    unsigned v0[kProbeSteps];
+    bool hit[kProbeSteps];
 #pragma unroll
-    for (int u = 0; u < kAhead; ++u) {
-      const unsigned m = __ballot_sync(0xffffffffu, key[u] != kEmptyKey && line[u] == key[u]);
+    for (int u = 0; u < kProbeSteps; ++u) {
+      const int w = key[u] != kEmptyKey ? match_tags(tags[u], key[u]) : -1;
+      const unsigned m = (__ballot_sync(kAll, w >= 0) >> (sub * kProbeLanes)) & ((1u << kProbeLanes) - 1u);
       hit[u] = m != 0;
-      slot[u] = set[u] * kWays + (hit[u] ? __ffs(m) - 1 : 0);
+      const int from = hit[u] ? __ffs(m) - 1 : 0;
+      const int way = __shfl_sync(kAll, l * 4 + (w < 0 ? 0 : w), from, kProbeLanes);
+      if (hit[u]) slot[u] += way;
       v0[u] = hit[u] ? *reinterpret_cast<volatile unsigned*>(&c.vers[slot[u]]) : 1u;
     }
     __threadfence();
+    unsigned long long k0[kProbeSteps];
 #pragma unroll
-    for (int u = 0; u < kAhead; ++u) {
-      if (!hit[u]) continue;
-      k0[u] = *reinterpret_cast<volatile unsigned long long*>(&c.keys[slot[u]]);
-      if (out != nullptr) copy_row_cg(out + (i0 + u * nwarps) * c.dim, c.values + slot[u] * c.dim, c.dim, lane);
+    for (int u = 0; u < kProbeSteps; ++u) {
+      k0[u] = kEmptyKey;
+      if (hit[u]) k0[u] = *reinterpret_cast<volatile unsigned long long*>(&c.keys[slot[u]]);
+    }
+    if (out != nullptr) {
+      // rows through L2, never from a possibly stale L1 line: the version check only vouches for what L2 holds
+      for (int v = l; v < (c.dim >> 2); v += kProbeLanes) {
+        float4 x[kProbeSteps];
+#pragma unroll
+        for (int u = 0; u < kProbeSteps; ++u)
+          if (hit[u]) x[u] = __ldcg(reinterpret_cast<const float4*>(c.values + slot[u] * c.dim) + v);
+#pragma unroll
+        for (int u = 0; u < kProbeSteps; ++u)
+          if (hit[u]) reinterpret_cast<float4*>(out + (i0 + u * (32 / kProbeLanes) + sub) * c.dim)[v] = x[u];
+      }
     }
     __threadfence();
+    bool my_miss = false;
 #pragma unroll
-    for (int u = 0; u < kAhead; ++u) {
-      if (key[u] == kEmptyKey) continue;                     // padding (or past the end): neither a hit nor a miss
+    for (int u = 0; u < kProbeSteps; ++u) {
       bool valid = false;
       if (hit[u]) {
         const unsigned v1 = *reinterpret_cast<volatile unsigned*>(&c.vers[slot[u]]);
-        valid = __all_sync(0xffffffffu, (v0[u] & 1u) == 0u && v1 == v0[u] && k0[u] == key[u]);
-        if (valid && lane == 0 && c.stamps[slot[u]] != now) c.stamps[slot[u]] = now;
+        valid = (v0[u] & 1u) == 0u && v1 == v0[u] && k0[u] == key[u];
       }
-      if (!valid) {
-        if (lane == n_miss) {
-          my_miss_index = i0 + u * nwarps;
-          my_miss_key = key[u];
-        }
-        if (++n_miss == 32) flush_misses();
+      // every lane of the key must have seen the same even version (they read it on their own)
+      const unsigned ok = (__ballot_sync(kAll, valid) >> (sub * kProbeLanes)) & ((1u << kProbeLanes) - 1u);
+      valid = ok == (1u << kProbeLanes) - 1u;
+      if (valid && l == 0 && c.stamps[slot[u]] != now) c.stamps[slot[u]] = now;
+      const int from = (lane - u * (32 / kProbeLanes)) * kProbeLanes;          // key `lane` was probed by these lanes
+      const bool theirs = __shfl_sync(kAll, static_cast<int>(valid), from & 31) != 0;
+      if (lane / (32 / kProbeLanes) == u) my_miss = !theirs && my_key != kEmptyKey;   // (padding: neither a hit nor a miss)
+    }
+    const unsigned misses = __ballot_sync(kAll, my_miss);
+    if (misses) {
+      int base = 0;
+      if (lane == 0) base = atomicAdd(miss_count, __popc(misses));
+      base = __shfl_sync(kAll, base, 0);
+      if (my_miss) {
+        const int at = base + __popc(misses & ((1u << lane) - 1u));
+        miss_index[at] = i0 + lane;
+        miss_keys[at] = static_cast<long long>(my_key);
       }
     }
   }
-  if (n_miss > 0) flush_misses();
 }
 
 __device__ __forceinline__ bool lock_set(int* lock, int lane) {
@@ -162,62 +183,90 @@ __device__ __forceinline__ void unlock_set(int* lock, int lane) {
 }
 
 // mode 0: Replace (insert or evict LRU, refresh stamp when present); mode 1: Update (present keys only).
+// Eight lanes per key, four keys per warp.  A write is a chain of about eight dependent memory round trips (lock, tags, version,
+// row, version, unlock and the fences between them), so what counts is how many keys are in such a chain at once: a warp per
+// key and 32 warps per SM took 81 us for 65,536 present keys x 32 floats.  Sets are locked by TRYING: a key whose set is
+// taken stays pending while the other keys of the warp go on, and no lane ever waits while it holds a lock.  The number of
+// tries is bounded; a key that never got its set is skipped and RS_DEV_WAIT_TIMEOUT recorded.
 __global__ void __launch_bounds__(256) cache_write_kernel(CacheView c, const long long* __restrict__ keys, long long n,
                                                           const float* __restrict__ values, int mode,
                                                           unsigned long long* status) {
-  const int lane = threadIdx.x & 31;
-  const long long warp = static_cast<long long>(blockIdx.x) * (blockDim.x >> 5) + (threadIdx.x >> 5);
+  constexpr unsigned kAll = 0xffffffffu;
+  constexpr int kPer = 32 / kProbeLanes;
+  const int lane = threadIdx.x & 31, l = lane & (kProbeLanes - 1), sub = lane / kProbeLanes;
+  const unsigned wm = ((1u << kProbeLanes) - 1u) << (sub * kProbeLanes);
   const long long nwarps = static_cast<long long>(gridDim.x) * (blockDim.x >> 5);
   const unsigned now = *c.clock;
-  for (long long i = warp; i < n; i += nwarps) {
-    const unsigned long long key = static_cast<unsigned long long>(keys[i]);
-    if (key == kEmptyKey) continue;
+  for (long long i0 = (static_cast<long long>(blockIdx.x) * (blockDim.x >> 5) + (threadIdx.x >> 5)) * kPer; i0 < n; i0 += nwarps * kPer) {
+    const long long i = i0 + sub;
+    const unsigned long long key = i < n ? static_cast<unsigned long long>(keys[i]) : kEmptyKey;
     const unsigned long long set = ht_hash(key) % c.nsets;
-    if (!lock_set(&c.locks[set], lane)) {
-      if (lane == 0 && status) atomicOr(status, (unsigned long long)RS_DEV_WAIT_TIMEOUT);
-      continue;
-    }
-    const unsigned long long line = *reinterpret_cast<volatile unsigned long long*>(&c.keys[set * kWays + lane]);
-    const unsigned hit = __ballot_sync(0xffffffffu, line == key);
-    int way = -1;
-    bool write_value = false;
-    if (hit) {
-      way = __ffs(hit) - 1;
-      write_value = (mode == 1);          // Replace of a cached key only refreshes its stamp
-    } else if (mode == 0) {
-      const unsigned empty = __ballot_sync(0xffffffffu, line == kEmptyKey);
-      if (empty) {
-        way = __ffs(empty) - 1;
-      } else {                             // evict the least recently stamped slot
-        unsigned st = *reinterpret_cast<volatile unsigned*>(&c.stamps[set * kWays + lane]);
-        unsigned long long best = (static_cast<unsigned long long>(st) << 5) | lane;
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
-          const unsigned long long other = __shfl_xor_sync(0xffffffffu, best, o);
-          best = other < best ? other : best;
-        }
-        way = static_cast<int>(best & 31);
-      }
-      write_value = true;
-    }
-    if (way >= 0) {
-      const unsigned long long slot = set * kWays + way;
-      if (write_value) {
-        // sequence number odd -> key and values change -> even again (readers discard what they copied meanwhile)
-        if (lane == 0) {
-          atomicAdd(&c.vers[slot], 1u);
-          __threadfence();
-        }
-        __syncwarp();
-        copy_row(c.values + slot * c.dim, values + i * c.dim, c.dim, lane);
-        if (lane == 0 && !hit) *reinterpret_cast<volatile unsigned long long*>(&c.keys[slot]) = key;
+    bool todo = key != kEmptyKey;
+    for (int spin = 0; spin < (1 << 20) && __any_sync(kAll, todo); ++spin) {
+      int got = 0;
+      if (todo && l == 0) got = atomicCAS(&c.locks[set], 0, 1) == 0;
+      got = __shfl_sync(kAll, got, 0, kProbeLanes);
+      if (got) {
+        todo = false;
         __threadfence();
-        __syncwarp();
-        if (lane == 0) atomicAdd(&c.vers[slot], 1u);
+        unsigned long long tags[4];
+        load_tags(tags, c.keys + set * kWays + l * 4);
+        const int w = match_tags(tags, key);
+        const unsigned hits = __ballot_sync(wm, w >= 0) >> (sub * kProbeLanes);
+        const bool hit = hits != 0;
+        int way = -1;
+        if (hit) {
+          way = __shfl_sync(wm, l * 4 + (w < 0 ? 0 : w), __ffs(hits) - 1, kProbeLanes);
+        } else if (mode == 0) {
+          // the first empty way, or the least recently stamped one
+          const int e = match_tags(tags, kEmptyKey);
+          const unsigned empty = __ballot_sync(wm, e >= 0) >> (sub * kProbeLanes);
+          if (empty) {
+            way = __shfl_sync(wm, l * 4 + (e < 0 ? 0 : e), __ffs(empty) - 1, kProbeLanes);
+          } else {
+            unsigned long long best = ~0ull;
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+              const unsigned st = *reinterpret_cast<volatile unsigned*>(&c.stamps[set * kWays + l * 4 + q]);
+              const unsigned long long mine = (static_cast<unsigned long long>(st) << 5) | static_cast<unsigned>(l * 4 + q);
+              best = mine < best ? mine : best;
+            }
+#pragma unroll
+            for (int o = kProbeLanes / 2; o > 0; o >>= 1) {
+              const unsigned long long other = __shfl_xor_sync(wm, best, o);
+              best = other < best ? other : best;
+            }
+            way = static_cast<int>(best & 31);
+          }
+        }
+        if (way >= 0) {
+          const unsigned long long slot = set * kWays + way;
+          if (!hit || mode == 1) {            // (Replace of a cached key only refreshes its stamp)
+            // sequence number odd -> key and values change -> even again (readers discard what they copied meanwhile)
+            if (l == 0) {
+              atomicAdd(&c.vers[slot], 1u);
+              __threadfence();
+            }
+            __syncwarp(wm);
+            for (int v = l; v < (c.dim >> 2); v += kProbeLanes)
+              reinterpret_cast<float4*>(c.values + slot * c.dim)[v] = reinterpret_cast<const float4*>(values + i * c.dim)[v];
+            if (l == 0 && !hit) *reinterpret_cast<volatile unsigned long long*>(&c.keys[slot]) = key;
+            __threadfence();
+            __syncwarp(wm);
+            if (l == 0) atomicAdd(&c.vers[slot], 1u);
+          }
+          if (l == 0 && mode == 0) c.stamps[slot] = now;
+        }
+        __syncwarp(wm);
+        if (l == 0) {
+          __threadfence();
+          atomicExch(&c.locks[set], 0);
+        }
       }
-      if (lane == 0 && mode == 0) c.stamps[slot] = now;
+      __syncwarp();
+      if (__any_sync(kAll, todo)) __nanosleep(32);
     }
-    unlock_set(&c.locks[set], lane);
+    if (todo && l == 0 && status) atomicOr(status, (unsigned long long)RS_DEV_WAIT_TIMEOUT);
   }
 }
 
@@ -418,8 +467,8 @@ RS_API int rs_cache_query(void* handle, const long long* keys, long long n, floa
   cache_tick_kernel<<<1, 1, 0, stream>>>(v.clock, miss_count);
   RS_LAUNCH_CHECK();
   if (n == 0) return RS_OK;
-  long long warps = (n + 3) / 4;  // >= 4 keys per warp when there are enough keys
-  if (warps > 148 * 24) warps = 148 * 24;    // three resident blocks of eight warps per SM (80 registers per thread)
+  long long warps = (n + kProbeKeys - 1) / kProbeKeys;
+  if (warps > 148 * 64) warps = 148 * 64;
   cache_query_kernel<<<static_cast<unsigned>((warps + 7) / 8), 256, 0, stream>>>(v, keys, n, out, miss_index, miss_keys, miss_count);
   RS_LAUNCH_CHECK();
   return RS_OK;
@@ -429,7 +478,9 @@ RS_API int rs_cache_replace(void* handle, const long long* keys, long long n, co
   RS_REQUIRE(handle && keys && values, "rs_cache_replace: null argument");
   if (n == 0) return RS_OK;
   CacheView& v = static_cast<CacheOwned*>(handle)->v;
-  long long warps = n < 148 * 32 ? n : 148 * 32;
+  const long long per = 32 / kProbeLanes;
+  long long warps = (n + per - 1) / per;
+  if (warps > 148 * 64) warps = 148 * 64;
   cache_write_kernel<<<static_cast<unsigned>((warps + 7) / 8), 256, 0, stream>>>(v, keys, n, values, 0, status);
   RS_LAUNCH_CHECK();
   return RS_OK;
@@ -439,7 +490,9 @@ RS_API int rs_cache_update(void* handle, const long long* keys, long long n, con
   RS_REQUIRE(handle && keys && values, "rs_cache_update: null argument");
   if (n == 0) return RS_OK;
   CacheView& v = static_cast<CacheOwned*>(handle)->v;
-  long long warps = n < 148 * 32 ? n : 148 * 32;
+  const long long per = 32 / kProbeLanes;
+  long long warps = (n + per - 1) / per;
+  if (warps > 148 * 64) warps = 148 * 64;
   cache_write_kernel<<<static_cast<unsigned>((warps + 7) / 8), 256, 0, stream>>>(v, keys, n, values, 1, status);
   RS_LAUNCH_CHECK();
   return RS_OK;
@@ -514,8 +567,8 @@ RS_API int rs_cache_query_noclock(void* handle, const long long* keys, long long
   CacheView& v = static_cast<CacheOwned*>(handle)->v;
   RS_CUDA(cudaMemsetAsync(miss_count, 0, sizeof(int), stream));
   if (n == 0) return RS_OK;
-  long long warps = (n + 3) / 4;
-  if (warps > 148 * 32) warps = 148 * 32;
+  long long warps = (n + kProbeKeys - 1) / kProbeKeys;
+  if (warps > 148 * 64) warps = 148 * 64;
   cache_query_kernel<<<static_cast<unsigned>((warps + 7) / 8), 256, 0, stream>>>(v, keys, n, out, miss_index, miss_keys, miss_count);
   RS_LAUNCH_CHECK();
   return RS_OK;
