@@ -419,6 +419,7 @@ class DLRM:
         self._pipe = bool(cfg.pipeline_lookup) and not self.dcn and not self.proj and not self.K
         self._pending: Optional[int] = None           # slot of the pending step
         self._launched = 0                            # steps whose graph has been launched
+        self._predicted = False                       # an inference pass has run
         self.s_wgrad = torch.cuda.Stream(device=dev, priority=p_wgrad)   # weight/bias gradients, then the dense all-reduce and SGD
         self.s_comm = torch.cuda.Stream(device=dev, priority=p_comm)     # embedding lookup / gradient push: the NVLink-bound kernels
         self.s_wgrad2 = torch.cuda.Stream(device=dev, priority=p_wgrad)  # weight gradients of the bottom MLP
@@ -894,10 +895,22 @@ class DLRM:
         with torch.cuda.graph(g, stream=torch.cuda.current_stream(), capture_error_mode="relaxed"):
             if mode == "lookup":
                 self._run_lookup(slot)
+            elif mode == "predict":
+                self._run_predict()
             else:
                 self._run_step(slot, mode)
         self._graphs[(slot, mode)] = g
         return g
+
+    def _run_predict(self):
+        self._no_stamp = True          # the phase stamps describe the last training step, not an inference pass
+        try:
+            x = self._forward(0)
+        finally:
+            self._no_stamp = False
+        F_.head_bce(x, self.head_w, self.head_b, None, 1.0 / self.B, prob=self.prob)
+        if self.world > 1:
+            self.ctx.barrier(CH_MISC)  # nobody may overwrite the interaction buffer before all have read it
 
     @torch.no_grad()
     def predict(self, batch: PinnedBatch) -> torch.Tensor:
@@ -908,14 +921,17 @@ class DLRM:
             self.in_ids[0].copy_(batch.ids, non_blocking=True)
             if self.K:
                 self.in_ids_rw[0].copy_(batch.ids_rw, non_blocking=True)
-            self._no_stamp = True          # the phase stamps describe the last training step, not an inference pass
-            try:
-                x = self._forward(0)
-            finally:
-                self._no_stamp = False
-            F_.head_bce(x, self.head_w, self.head_b, None, 1.0 / self.B, prob=self.prob)
-            if self.world > 1:
-                self.ctx.barrier(CH_MISC)  # nobody may overwrite the interaction buffer before all have read it
+            # A request of some hundred samples is a dozen kernels of a few microseconds each, which the host cannot launch as
+            # fast as they run (198 us a call at 1,000 samples, 40 us of it on the device): from the second call on the pass
+            # is replayed as a graph.  The first call runs eagerly: a capture costs more than it saves to whoever calls once.
+            if self.cfg.use_cuda_graph and self._predicted:
+                g = self._graphs.get((0, "predict"))
+                if g is None:
+                    g = self._capture(0, "predict")
+                g.replay()
+            else:
+                self._run_predict()
+                self._predicted = True
             out = self.prob.clone()
         self.compute_stream.synchronize()
         return out
