@@ -118,22 +118,32 @@ template <int V> __device__ __forceinline__ void row_atomic_add(float* p, const 
   for (int e = 0; e < V; e += 4) atomicAdd(reinterpret_cast<float4*>(p + e), make_float4(r.v[e], r.v[e + 1], r.v[e + 2], r.v[e + 3]));
 }
 
-// Sum of `v` over the lanes of the warp that hold the same `key`, valid in the lowest of them (returned as true).  Equal lanes
-// form a chain in lane order that halves with every step; a warp without duplicates leaves after one vote.
-__device__ __forceinline__ bool warp_sum_equal_keys(unsigned long long key, float& v) {
+// peers[r]: the lanes that hold the same key as this one (__match_any_sync).  Leaves in the lowest lane of every such set the
+// sum of its v[r].  Equal lanes form a chain in lane order that halves with every step; the R chains step together, and a
+// warp without duplicates leaves after one vote.
+template <int R>
+__device__ __forceinline__ void warp_sum_peers(const unsigned (&peers)[R], float (&v)[R]) {
   const int lane = threadIdx.x & 31;
-  const unsigned peers = __match_any_sync(0xffffffffu, key);
-  const unsigned above = peers & (0xfffffffeu << lane);
-  int next = above ? __ffs(above) - 1 : -1;
+  int next[R];
+#pragma unroll
+  for (int r = 0; r < R; ++r) {
+    const unsigned above = peers[r] & (0xfffffffeu << lane);
+    next[r] = above ? __ffs(above) - 1 : -1;
+  }
 #pragma unroll
   for (int s = 0; s < 5; ++s) {
-    if (__all_sync(0xffffffffu, next < 0)) break;
-    const int from = next < 0 ? lane : next;
-    const float o = __shfl_sync(0xffffffffu, v, from);
-    const int n2 = __shfl_sync(0xffffffffu, next, from);
-    if (next >= 0) { v += o; next = n2; }
+    bool done = true;
+#pragma unroll
+    for (int r = 0; r < R; ++r) done = done && next[r] < 0;
+    if (__all_sync(0xffffffffu, done)) break;
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+      const int from = next[r] < 0 ? lane : next[r];
+      const float o = __shfl_sync(0xffffffffu, v[r], from);
+      const int n2 = __shfl_sync(0xffffffffu, next[r], from);
+      if (next[r] >= 0) { v[r] += o; next[r] = n2; }
+    }
   }
-  return lane == __ffs(peers) - 1;
 }
 
 // Chooses <V, L, NC> for rows of D floats; `wide`: D is a multiple of 8 and every row starts on a 32-byte boundary.

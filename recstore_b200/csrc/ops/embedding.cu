@@ -440,8 +440,9 @@ __device__ __forceinline__ long long live_nnz(const EmbBwdArgs& a) {
 }
 
 constexpr int kStateMax = 1024;  // occurrences a CTA of the state pass folds
-constexpr int kApplyThreads = 512;
-constexpr int kApplyMax = 1024;  // occurrences a CTA of the apply pass sorts
+constexpr int kApplyThreads = 512;   // threads of an apply CTA (128 in small batches) ...
+constexpr int kApplyPer = 2;     // ... and the occurrences each of them takes at most
+constexpr int kApplyMax = kApplyThreads * kApplyPer;
 
 // Sample and table of occurrence i.  32-bit arithmetic wherever the bag number allows it: a 64-bit division costs more
 // than the rest of the address computation.
@@ -476,10 +477,22 @@ __device__ __forceinline__ void state_fold_clear(StateFold& f, int slots) {
   }
   __syncthreads();
 }
-// All lanes of a warp; row < 0: nothing to add.
-__device__ __forceinline__ void state_fold_add(StateFold& f, int slots, long long row, float v) {
-  const bool first = rs::warp_sum_equal_keys(static_cast<unsigned long long>(row), v);
-  if (!first || row < 0) return;
+// One value per lane and round of a warp, summed over equal rows and added to the fold; row < 0: nothing to add.
+// `narrow`: rows fit into 32 bits (the match of 64-bit values costs twice as much).
+__device__ __forceinline__ void state_fold_insert(StateFold& f, int slots, long long row, float v);
+template <int R>
+__device__ __forceinline__ void state_fold_add(StateFold& f, int slots, const long long (&row)[R], float (&v)[R], bool narrow) {
+  unsigned peers[R];
+#pragma unroll
+  for (int r = 0; r < R; ++r)
+    peers[r] = narrow ? __match_any_sync(0xffffffffu, static_cast<unsigned>(row[r]))
+                      : __match_any_sync(0xffffffffu, static_cast<unsigned long long>(row[r]));
+  rs::warp_sum_peers(peers, v);
+#pragma unroll
+  for (int r = 0; r < R; ++r)
+    if (row[r] >= 0 && static_cast<int>(threadIdx.x & 31) == __ffs(peers[r]) - 1) state_fold_insert(f, slots, row[r], v[r]);
+}
+__device__ __forceinline__ void state_fold_insert(StateFold& f, int slots, long long row, float v) {
   unsigned s = static_cast<unsigned>(rs::ht_hash(static_cast<unsigned long long>(row))) & (slots - 1);
   for (int p = 0; p < slots; ++p) {
     const unsigned long long prev = atomicCAS(&f.key[s], ~0ull, static_cast<unsigned long long>(row));
@@ -525,9 +538,14 @@ __global__ void __launch_bounds__(256) emb_state_norm_kernel(const EmbBwdArgs a,
       }
     }
   }
-#pragma unroll
-  for (int r = 0; r < 4; ++r)
-    if (r < rounds) state_fold_add(f, slots, row[r], v[r]);
+  const bool narrow = a.total_rows < 0xffffffffll;
+  if (rounds > 1) {
+    state_fold_add(f, slots, row, v, narrow);
+  } else {
+    const long long row1[1] = {row[0]};
+    float v1[1] = {v[0]};
+    state_fold_add(f, slots, row1, v1, narrow);
+  }
   state_fold_flush(f, slots, a.state);
 }
 
@@ -596,8 +614,9 @@ __global__ void __launch_bounds__(256) emb_state_kernel(const EmbBwdArgs a, cons
         if (k >= 0 && k < G) v = got;
       }
     }
-    v *= w * w / static_cast<float>(a.D);
-    state_fold_add(f, slots, row, v);
+    const long long row1[1] = {row};
+    float v1[1] = {v * (w * w / static_cast<float>(a.D))};
+    state_fold_add(f, slots, row1, v1, a.total_rows < 0xffffffffll);
   }
   state_fold_flush(f, slots, a.state);
 }
@@ -614,11 +633,11 @@ __global__ void __launch_bounds__(256) emb_state_kernel(const EmbBwdArgs a, cons
 // 278 us for 1.70 M occurrences x 128 at Zipf 1.2.
 template <int V, int L, int NC, bool BF16>
 __global__ void __launch_bounds__(kApplyThreads) emb_apply_kernel(const EmbBwdArgs a, const int gs) {
-  constexpr int kPer = kApplyMax / kApplyThreads;
-  constexpr int kWarps = kApplyThreads / 32;
+  constexpr int kPer = kApplyPer;
+  const int threads = blockDim.x, warps = threads >> 5;
   // the hash is dead once the positions are known; the sorted arrays take its place
   __shared__ __align__(16) unsigned char s_mem[2 * kApplyMax * 12 > kApplyMax * 20 ? 2 * kApplyMax * 12 : kApplyMax * 20];
-  __shared__ int s_warp_sum[kWarps];
+  __shared__ int s_warp_sum[kApplyThreads / 32];
   long long* const s_key = reinterpret_cast<long long*>(s_mem);                        // [2 gs]
   int* const s_cnt = reinterpret_cast<int*>(s_mem + 2 * kApplyMax * 8);                // [2 gs] occurrences per slot, then offsets
   long long* const s_goff = reinterpret_cast<long long*>(s_mem);                       // sorted: gradient offset
@@ -632,7 +651,7 @@ __global__ void __launch_bounds__(kApplyThreads) emb_apply_kernel(const EmbBwdAr
   if (g0 >= nnz) return;                       // whole group past the live occurrences
   rs::flag_wait_all(a.wait);
   const int slots = 2 * gs;
-  for (int s = tid; s < slots; s += kApplyThreads) {
+  for (int s = tid; s < slots; s += threads) {
     s_key[s] = -1;
     s_cnt[s] = 0;
   }
@@ -641,7 +660,7 @@ __global__ void __launch_bounds__(kApplyThreads) emb_apply_kernel(const EmbBwdAr
   bool narrow = false;
 #pragma unroll
   for (int q = 0; q < kPer; ++q) {
-    const int at = q * kApplyThreads + tid;
+    const int at = q * threads + tid;
     row[q] = -1;
     goff[q] = 0;
     coef[q] = -a.lr;
@@ -656,7 +675,7 @@ __global__ void __launch_bounds__(kApplyThreads) emb_apply_kernel(const EmbBwdAr
 #pragma unroll
   for (int q = 0; q < kPer; ++q) {
     if (row[q] < 0) continue;
-    const long long occ = g0 + q * kApplyThreads + tid;
+    const long long occ = g0 + q * threads + tid;
     int t, b;
     bag_of(a, occ, t, b);
     goff[q] = b * a.grad_row_stride + (a.grad_col ? a.grad_col[t] : 0);
@@ -704,8 +723,7 @@ __global__ void __launch_bounds__(kApplyThreads) emb_apply_kernel(const EmbBwdAr
     if (lane == 31) s_warp_sum[warp] = incl;
     __syncthreads();
     int excl = incl - sum;
-#pragma unroll
-    for (int q = 0; q < kWarps; ++q) {
+    for (int q = 0; q < warps; ++q) {
       excl += q < warp ? s_warp_sum[q] : 0;
       total += s_warp_sum[q];
     }
@@ -733,7 +751,7 @@ __global__ void __launch_bounds__(kApplyThreads) emb_apply_kernel(const EmbBwdAr
   constexpr int U = V * NC <= 8 ? 4 : 2;
   const int l = lane & (L - 1);
   const int nvec = a.D / V;
-  const int share = gs / (kWarps * G);
+  const int share = gs / (warps * G);
   const int p_begin = (warp * G + lane / L) * share;
   const int p_end = min(total, p_begin + share);
   long long cur = -1;
@@ -1022,11 +1040,13 @@ int emb_backward_impl(float* weight, float* state, long long total_rows, const l
     }
     RS_LAUNCH_CHECK();
   }
-  // The largest group that still gives every SM two CTAs, never less than one position per sub-warp.
+  // The largest group that still gives every SM two CTAs, never less than one position per sub-warp.  CTAs of 512 threads
+  // once a batch fills them; below, the barriers of the sort cost more than the warps gain (3,072 rows of 400: 15.5 us).
   auto launch = [&](auto kern, int L) {
-    int gs = kApplyMax;
-    while (gs > (kApplyThreads / 32) * (32 / L) && nnz < 296ll * gs) gs >>= 1;
-    kern<<<static_cast<unsigned>((nnz + gs - 1) / gs), kApplyThreads, 0, stream>>>(a, gs);
+    const int threads = nnz >= 296ll * kApplyThreads ? kApplyThreads : 128;
+    int gs = threads * kApplyPer;
+    while (gs > (threads / 32) * (32 / L) && nnz < 296ll * gs) gs >>= 1;
+    kern<<<static_cast<unsigned>((nnz + gs - 1) / gs), threads, 0, stream>>>(a, gs);
   };
 #define RS_LAUNCH_APPLY(V, L, NC)                                 \
   do {                                                            \
