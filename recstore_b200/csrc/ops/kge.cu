@@ -106,6 +106,57 @@ __device__ __forceinline__ float pair_psi(int model, float d0, float d1, float& 
   u0 = d0 * inv; u1 = d1 * inv;
   return m2 * inv;
 }
+// The loops over the pairs work on TWO rows at once in packed fp32 (f32x2): they are bound by issue slots, and a packed
+// instruction does the same correctly rounded operation on both halves in one slot.
+typedef unsigned long long f32x2;
+__device__ __forceinline__ f32x2 pack2(float lo, float hi) {
+  f32x2 r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
+  return r;
+}
+__device__ __forceinline__ void unpack2(f32x2 v, float& lo, float& hi) { asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v)); }
+__device__ __forceinline__ f32x2 add2(f32x2 a, f32x2 b) {
+  f32x2 r;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ f32x2 mul2(f32x2 a, f32x2 b) {
+  f32x2 r;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) {
+  f32x2 r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+  return r;
+}
+// (g0, g1) += w * d psi / d difference.  RotatE: the lower bound only keeps 0 * (1 / 0) out.
+__device__ __forceinline__ void pair_pull(int model, f32x2 d0, f32x2 d1, f32x2 w, f32x2& g0, f32x2& g1) {
+  if (model == kTransE1) {
+    float a, b;
+    unpack2(d0, a, b);
+    g0 = fma2(w, pack2(sgn(a), sgn(b)), g0);
+    unpack2(d1, a, b);
+    g1 = fma2(w, pack2(sgn(a), sgn(b)), g1);
+  } else {
+    float a, b;
+    unpack2(fma2(d1, d1, mul2(d0, d0)), a, b);
+    const f32x2 c = mul2(w, pack2(rsqrtf(fmaxf(a, 1e-37f)), rsqrtf(fmaxf(b, 1e-37f))));
+    g0 = fma2(c, d0, g0);
+    g1 = fma2(c, d1, g1);
+  }
+}
+__device__ __forceinline__ f32x2 pair_dist2(int model, f32x2 d0, f32x2 d1) {
+  float a, b;
+  if (model == kTransE1) {
+    float c, d;
+    unpack2(d0, a, b);
+    unpack2(d1, c, d);
+    return add2(pack2(fabsf(a), fabsf(b)), pack2(fabsf(c), fabsf(d)));
+  }
+  unpack2(fma2(d1, d1, mul2(d0, d0)), a, b);
+  return pack2(sqrtf(a), sqrtf(b));
+}
 __device__ __forceinline__ float pair_dist(int model, float d0, float d1) {
   return model == kTransE1 ? fabsf(d0) + fabsf(d1) : sqrtf(d0 * d0 + d1 * d1);
 }
@@ -348,17 +399,30 @@ __global__ void __launch_bounds__(256) kge_prepare_kernel(const KgeArgs k) {
   const float to_phase = kPi / k.emb_init;
   float* A32 = k.A32 + static_cast<size_t>(i) * k.Dp;
   float dist = 0.f;
-  for (int kk = lane; kk < H; kk += 32) {
-    float a0, a1;
-    if (k.model == kTransE1) {
-      a0 = x[kk] + sg * r[kk]; a1 = x[kk + H] + sg * r[kk + H];
-    } else {
-      float sn, c;
-      __sincosf(r[kk] * to_phase, &sn, &c);
-      a0 = x[kk] * c - sg * x[kk + H] * sn; a1 = sg * x[kk] * sn + x[kk + H] * c;
+  const bool l1 = k.model == kTransE1;
+  for (int kk0 = lane; kk0 < H; kk0 += 32 * kRowBatch) {           // loads of kRowBatch elements before the first is used
+    float x0[kRowBatch], x1[kRowBatch], y0[kRowBatch], y1[kRowBatch], r0[kRowBatch], r1[kRowBatch];
+#pragma unroll
+    for (int u = 0; u < kRowBatch; ++u) {
+      const int kk = min(kk0 + 32 * u, H - 1);
+      x0[u] = x[kk]; x1[u] = x[kk + H]; y0[u] = y[kk]; y1[u] = y[kk + H];
+      r0[u] = r[kk]; r1[u] = l1 ? r[kk + H] : 0.f;
     }
-    A32[kk] = a0; A32[kk + H] = a1;
-    dist += pair_dist(k.model, a0 - y[kk], a1 - y[kk + H]);
+#pragma unroll
+    for (int u = 0; u < kRowBatch; ++u) {
+      const int kk = kk0 + 32 * u;
+      if (kk >= H) break;
+      float a0, a1;
+      if (l1) {
+        a0 = x0[u] + sg * r0[u]; a1 = x1[u] + sg * r1[u];
+      } else {
+        float sn, c;
+        __sincosf(r0[u] * to_phase, &sn, &c);
+        a0 = x0[u] * c - sg * x1[u] * sn; a1 = sg * x0[u] * sn + x1[u] * c;
+      }
+      A32[kk] = a0; A32[kk + H] = a1;
+      dist += pair_dist(k.model, a0 - y0[u], a1 - y1[u]);
+    }
   }
   dist = warp_sum(dist);
   const float score = k.gamma - dist;
@@ -368,10 +432,21 @@ __global__ void __launch_bounds__(256) kge_prepare_kernel(const KgeArgs k) {
     if (k.pos_score) k.pos_score[i] = score;
     atomicAdd(&k.loss[0], -log_sigmoid(score) * inv_bs);
   }
-  for (int kk = lane; kk < H; kk += 32) {            // d loss / d y = q * (-1) * (-u)
-    float u0, u1;
-    pair_psi(k.model, A32[kk] - y[kk], A32[kk + H] - y[kk + H], u0, u1);
-    gy[kk] = q * u0; gy[kk + H] = q * u1;
+  for (int kk0 = lane; kk0 < H; kk0 += 32 * kRowBatch) {           // d loss / d y = q * (-1) * (-u)
+    float d0[kRowBatch], d1[kRowBatch];
+#pragma unroll
+    for (int u = 0; u < kRowBatch; ++u) {
+      const int kk = min(kk0 + 32 * u, H - 1);
+      d0[u] = A32[kk] - y[kk]; d1[u] = A32[kk + H] - y[kk + H];
+    }
+#pragma unroll
+    for (int u = 0; u < kRowBatch; ++u) {
+      const int kk = kk0 + 32 * u;
+      if (kk >= H) break;
+      float u0, u1;
+      pair_psi(k.model, d0[u], d1[u], u0, u1);
+      gy[kk] = q * u0; gy[kk + H] = q * u1;
+    }
   }
 }
 
@@ -603,7 +678,8 @@ __global__ void __launch_bounds__(256) kge_finish_kernel(const KgeArgs k) {
 // (114 registers, 23 % of the warps resident, 53 us for 1,024 x 256 pairs of 200 complex elements).
 constexpr int kPairTileI = 4, kPairTileJ = 4;
 template <int MODEL>
-__global__ void __launch_bounds__(256, 4) kge_pair_forward_kernel(const KgeArgs k) {
+__global__ void __launch_bounds__(256, 3) kge_pair_forward_kernel(const KgeArgs k) {
+  __shared__ float s_l[8];
   const int lane = threadIdx.x & 31;
   const int warp = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   const int jt = k.ns / kPairTileJ;                // tiles of negatives per chunk
@@ -615,20 +691,38 @@ __global__ void __launch_bounds__(256, 4) kge_pair_forward_kernel(const KgeArgs 
     const int H = k.D >> 1;
     const float* a = k.A32 + static_cast<size_t>(i0) * k.Dp;
     const float* n = k.neg + (static_cast<size_t>(c) * k.ns + j0) * k.D;
-    float v[16];
+    f32x2 v2[2][4];                                // positives 2 q and 2 q + 1 against negative jj
 #pragma unroll
-    for (int p = 0; p < 16; ++p) v[p] = 0.f;
-    for (int kk = lane; kk < H; kk += 32) {
-      float a0[4], a1[4], n0[4], n1[4];
+    for (int q = 0; q < 2; ++q)
+#pragma unroll
+      for (int jj = 0; jj < 4; ++jj) v2[q][jj] = 0ull;
+    // The operands of the next step are fetched while this one's pairs are worked out; past the end the last are fetched again.
+    float a0[4], a1[4], n0[4], n1[4];
+    auto fetch = [&](int kk) {
+      kk = min(kk, H - 1);
 #pragma unroll
       for (int ii = 0; ii < 4; ++ii) { a0[ii] = a[ii * k.Dp + kk]; a1[ii] = a[ii * k.Dp + kk + H]; }
 #pragma unroll
       for (int jj = 0; jj < 4; ++jj) { n0[jj] = n[jj * k.D + kk]; n1[jj] = n[jj * k.D + kk + H]; }
+    };
+    fetch(lane);
+    for (int kk = lane; kk < H; kk += 32) {
+      f32x2 b0[2], b1[2], m0[4], m1[4];
 #pragma unroll
-      for (int ii = 0; ii < 4; ++ii)
+      for (int q = 0; q < 2; ++q) { b0[q] = pack2(a0[2 * q], a0[2 * q + 1]); b1[q] = pack2(a1[2 * q], a1[2 * q + 1]); }
 #pragma unroll
-        for (int jj = 0; jj < 4; ++jj) v[ii * 4 + jj] += pair_dist(MODEL, a0[ii] - n0[jj], a1[ii] - n1[jj]);
+      for (int jj = 0; jj < 4; ++jj) { m0[jj] = pack2(-n0[jj], -n0[jj]); m1[jj] = pack2(-n1[jj], -n1[jj]); }
+      fetch(kk + 32);
+#pragma unroll
+      for (int q = 0; q < 2; ++q)
+#pragma unroll
+        for (int jj = 0; jj < 4; ++jj) v2[q][jj] = add2(v2[q][jj], pair_dist2(MODEL, add2(b0[q], m0[jj]), add2(b1[q], m1[jj])));
     }
+    float v[16];
+#pragma unroll
+    for (int q = 0; q < 2; ++q)
+#pragma unroll
+      for (int jj = 0; jj < 4; ++jj) unpack2(v2[q][jj], v[8 * q + jj], v[8 * q + 4 + jj]);
 #pragma unroll
     for (int o = 16, cnt = 16; o > 1; o >>= 1, cnt >>= 1) {
       const bool upper = (lane & o) != 0;
@@ -650,24 +744,33 @@ __global__ void __launch_bounds__(256, 4) kge_pair_forward_kernel(const KgeArgs 
       l = -log_sigmoid(-score) * norm;
     }
   }
+  // one atomic per block: a chain of fewer and larger terms is also the more exact sum
   l = warp_sum(l);
-  if (lane == 0 && l != 0.f) atomicAdd(&k.loss[1], l);
+  if (lane == 0) s_l[threadIdx.x >> 5] = l;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    l = 0.f;
+#pragma unroll
+    for (int q = 0; q < 8; ++q) l += s_l[q];
+    if (l != 0.f) atomicAdd(&k.loss[1], l);
+  }
 }
 
 constexpr int kPairRows = 8;      // rows that share one pass over the other side
 constexpr int kPairTile = 256;    // weights staged per pass
-constexpr int kPairCols = 64;     // element pairs per block
-constexpr int kPairWays = 4;      // threads that share an element pair, each walking its part of the other side
+constexpr int kPairCols = 32;     // element pairs per block: a warp per way
+constexpr int kPairWays = 4;      // warps that share an element pair, each walking its part of the other side
 constexpr int kPairThreads = kPairCols * kPairWays;
-constexpr int kPairBatch = 4;     // rows of the other side a thread fetches at once
+constexpr int kPairBatch = 2;     // rows of the other side a thread fetches at once
 
 // Sums the kPairWays partial gradients of every element pair into the threads of way 0.
-__device__ __forceinline__ void pair_join(float (&g0)[kPairRows], float (&g1)[kPairRows], float* buf, int col, int way) {
+__device__ __forceinline__ void pair_join(f32x2 (&g0)[kPairRows / 2], f32x2 (&g1)[kPairRows / 2], float* mem, int col, int way) {
+  f32x2* buf = reinterpret_cast<f32x2*>(mem);
   for (int q = 1; q < kPairWays; ++q) {
     __syncthreads();
     if (way == q) {
 #pragma unroll
-      for (int rr = 0; rr < kPairRows; ++rr) {
+      for (int rr = 0; rr < kPairRows / 2; ++rr) {
         buf[(2 * rr) * kPairCols + col] = g0[rr];
         buf[(2 * rr + 1) * kPairCols + col] = g1[rr];
       }
@@ -675,35 +778,37 @@ __device__ __forceinline__ void pair_join(float (&g0)[kPairRows], float (&g1)[kP
     __syncthreads();
     if (way == 0) {
 #pragma unroll
-      for (int rr = 0; rr < kPairRows; ++rr) {
-        g0[rr] += buf[(2 * rr) * kPairCols + col];
-        g1[rr] += buf[(2 * rr + 1) * kPairCols + col];
+      for (int rr = 0; rr < kPairRows / 2; ++rr) {
+        g0[rr] = add2(g0[rr], buf[(2 * rr) * kPairCols + col]);
+        g1[rr] = add2(g1[rr], buf[(2 * rr + 1) * kPairCols + col]);
       }
     }
   }
 }
 
-// The two gradient kernels: a block owns 8 rows of one side x 64 element pairs; its 4 ways of threads walk a quarter of the
+// The two gradient kernels: a block owns 8 rows of one side x 32 element pairs; its 4 warps walk a quarter of the
 // other side's rows of the chunk each and add up at the end, so every gradient element still has one owner and no atomics.
 // Bound by issue slots (about a dozen instructions and one special function per element of a pair); one way of 128 threads
 // left three quarters of the warps out: 167 and 159 us for 1,024 x 256 pairs of 200 complex elements, 9 % resident.
 
 // Block = 8 positives of one chunk; chains d loss / d a (negatives and the positive) to x and r.
 template <int MODEL>
-__global__ void __launch_bounds__(kPairThreads) kge_pair_grad_pos_kernel(const KgeArgs k) {
-  __shared__ __align__(16) float w[kPairTile][kPairRows];      // (the join's 16 x 64 floats fit into it)
+__global__ void __launch_bounds__(kPairThreads, 8) kge_pair_grad_pos_kernel(const KgeArgs k) {
+  __shared__ __align__(16) float w[kPairTile][kPairRows];      // (the join's 8 x 32 packed pairs fit into it)
   const int i0 = blockIdx.x * kPairRows;
   const int c = i0 / k.cs;
   const int H = k.D >> 1;
   const int col = threadIdx.x % kPairCols, way = threadIdx.x / kPairCols;
   const int kk = blockIdx.y * kPairCols + col;
   const bool live = kk < H;
-  float a0[kPairRows], a1[kPairRows], g0[kPairRows], g1[kPairRows];
+  f32x2 a0[kPairRows / 2], a1[kPairRows / 2], g0[kPairRows / 2], g1[kPairRows / 2];   // rows 2 q and 2 q + 1
 #pragma unroll
-  for (int rr = 0; rr < kPairRows; ++rr) {
-    a0[rr] = live ? k.A32[static_cast<size_t>(i0 + rr) * k.Dp + kk] : 0.f;
-    a1[rr] = live ? k.A32[static_cast<size_t>(i0 + rr) * k.Dp + kk + H] : 0.f;
-    g0[rr] = 0.f; g1[rr] = 0.f;
+  for (int q = 0; q < kPairRows / 2; ++q) {
+    const float* lo = k.A32 + static_cast<size_t>(i0 + 2 * q) * k.Dp;
+    const float* hi = lo + k.Dp;
+    a0[q] = live ? pack2(lo[kk], hi[kk]) : 0ull;
+    a1[q] = live ? pack2(lo[kk + H], hi[kk + H]) : 0ull;
+    g0[q] = 0ull; g1[q] = 0ull;
   }
   for (int jb = 0; jb < k.ns; jb += kPairTile) {
     const int nj = min(kPairTile, k.ns - jb);
@@ -727,14 +832,11 @@ __global__ void __launch_bounds__(kPairThreads) kge_pair_grad_pos_kernel(const K
         for (int q = 0; q < kPairBatch; ++q) {
           const int j = jj0 + q * kPairWays;
           if (j >= nj) break;
-          const float4 wa = *reinterpret_cast<const float4*>(&w[j][0]), wb = *reinterpret_cast<const float4*>(&w[j][4]);
-          const float ww[kPairRows] = {wa.x, wa.y, wa.z, wa.w, wb.x, wb.y, wb.z, wb.w};
+          const ulonglong2 wa = *reinterpret_cast<const ulonglong2*>(&w[j][0]), wb = *reinterpret_cast<const ulonglong2*>(&w[j][4]);
+          const f32x2 ww[kPairRows / 2] = {wa.x, wa.y, wb.x, wb.y};
+          const f32x2 m0 = pack2(-n0[q], -n0[q]), m1 = pack2(-n1[q], -n1[q]);
 #pragma unroll
-          for (int rr = 0; rr < kPairRows; ++rr) {
-            float u0, u1;
-            pair_psi(MODEL, a0[rr] - n0[q], a1[rr] - n1[q], u0, u1);
-            g0[rr] -= ww[rr] * u0; g1[rr] -= ww[rr] * u1;
-          }
+          for (int rr = 0; rr < kPairRows / 2; ++rr) pair_pull(MODEL, add2(a0[rr], m0), add2(a1[rr], m1), ww[rr], g0[rr], g1[rr]);
         }
       }
     }
@@ -751,10 +853,14 @@ __global__ void __launch_bounds__(kPairThreads) kge_pair_grad_pos_kernel(const K
     const float* y = (ch ? k.h : k.t) + static_cast<size_t>(i) * k.D;
     float* gx = (ch ? k.gt : k.gh) + static_cast<size_t>(i) * k.D;
     float* gr = k.gr + static_cast<size_t>(i) * k.Dr;
-    float u0, u1;
-    pair_psi(MODEL, a0[rr] - y[kk], a1[rr] - y[kk + H], u0, u1);
+    float u0, u1, p0[2], p1[2], s0[2], s1[2];
+    unpack2(a0[rr / 2], p0[0], p0[1]);
+    unpack2(a1[rr / 2], p1[0], p1[1]);
+    unpack2(g0[rr / 2], s0[0], s0[1]);
+    unpack2(g1[rr / 2], s1[0], s1[1]);
+    pair_psi(MODEL, p0[rr & 1] - y[kk], p1[rr & 1] - y[kk + H], u0, u1);
     const float q = k.a2[i];
-    const float ga0 = g0[rr] - q * u0, ga1 = g1[rr] - q * u1;
+    const float ga0 = -s0[rr & 1] - q * u0, ga1 = -s1[rr & 1] - q * u1;     // (d loss / d dist = -w)
     if (MODEL == kTransE1) {
       gx[kk] = ga0; gx[kk + H] = ga1; gr[kk] = sg * ga0; gr[kk + H] = sg * ga1;
     } else {
@@ -771,7 +877,7 @@ __global__ void __launch_bounds__(kPairThreads) kge_pair_grad_pos_kernel(const K
 
 // Block = 8 negatives of one chunk; its threads walk the chunk's positives.
 template <int MODEL>
-__global__ void __launch_bounds__(kPairThreads) kge_pair_grad_neg_kernel(const KgeArgs k) {
+__global__ void __launch_bounds__(kPairThreads, 8) kge_pair_grad_neg_kernel(const KgeArgs k) {
   __shared__ __align__(16) float w[kPairTile][kPairRows];
   const int col0 = blockIdx.x * kPairRows;          // index into [C*ns]
   const int c = col0 / k.ns, j0 = col0 - c * k.ns;
@@ -779,12 +885,14 @@ __global__ void __launch_bounds__(kPairThreads) kge_pair_grad_neg_kernel(const K
   const int col = threadIdx.x % kPairCols, way = threadIdx.x / kPairCols;
   const int kk = blockIdx.y * kPairCols + col;
   const bool live = kk < H;
-  float n0[kPairRows], n1[kPairRows], g0[kPairRows], g1[kPairRows];
+  f32x2 n0[kPairRows / 2], n1[kPairRows / 2], g0[kPairRows / 2], g1[kPairRows / 2];   // minus rows 2 q and 2 q + 1
 #pragma unroll
-  for (int jj = 0; jj < kPairRows; ++jj) {
-    n0[jj] = live ? k.neg[static_cast<size_t>(col0 + jj) * k.D + kk] : 0.f;
-    n1[jj] = live ? k.neg[static_cast<size_t>(col0 + jj) * k.D + kk + H] : 0.f;
-    g0[jj] = 0.f; g1[jj] = 0.f;
+  for (int q = 0; q < kPairRows / 2; ++q) {
+    const float* lo = k.neg + static_cast<size_t>(col0 + 2 * q) * k.D;
+    const float* hi = lo + k.D;
+    n0[q] = live ? pack2(-lo[kk], -hi[kk]) : 0ull;
+    n1[q] = live ? pack2(-lo[kk + H], -hi[kk + H]) : 0ull;
+    g0[q] = 0ull; g1[q] = 0ull;
   }
   for (int ib = 0; ib < k.cs; ib += kPairTile) {
     const int ni = min(kPairTile, k.cs - ib);
@@ -807,14 +915,12 @@ __global__ void __launch_bounds__(kPairThreads) kge_pair_grad_neg_kernel(const K
         for (int q = 0; q < kPairBatch; ++q) {
           const int ii = ii0 + q * kPairWays;
           if (ii >= ni) break;
-          const float4 wa = *reinterpret_cast<const float4*>(&w[ii][0]), wb = *reinterpret_cast<const float4*>(&w[ii][4]);
-          const float ww[kPairRows] = {wa.x, wa.y, wa.z, wa.w, wb.x, wb.y, wb.z, wb.w};
+          const ulonglong2 wa = *reinterpret_cast<const ulonglong2*>(&w[ii][0]), wb = *reinterpret_cast<const ulonglong2*>(&w[ii][4]);
+          const f32x2 ww[kPairRows / 2] = {wa.x, wa.y, wb.x, wb.y};
+          const f32x2 p0 = pack2(a0[q], a0[q]), p1 = pack2(a1[q], a1[q]);
 #pragma unroll
-          for (int jj = 0; jj < kPairRows; ++jj) {
-            float u0, u1;
-            pair_psi(MODEL, a0[q] - n0[jj], a1[q] - n1[jj], u0, u1);
-            g0[jj] += ww[jj] * u0; g1[jj] += ww[jj] * u1;     // d loss / d dist = -w, d dist / d e' = -u
-          }
+          for (int jj = 0; jj < kPairRows / 2; ++jj)      // d loss / d dist = -w, d dist / d e' = -u
+            pair_pull(MODEL, add2(p0, n0[jj]), add2(p1, n1[jj]), ww[jj], g0[jj], g1[jj]);
         }
       }
     }
@@ -822,9 +928,11 @@ __global__ void __launch_bounds__(kPairThreads) kge_pair_grad_neg_kernel(const K
   pair_join(g0, g1, &w[0][0], col, way);
   if (!live || way != 0) return;
 #pragma unroll
-  for (int jj = 0; jj < kPairRows; ++jj) {
-    k.gneg[static_cast<size_t>(col0 + jj) * k.D + kk] = g0[jj];
-    k.gneg[static_cast<size_t>(col0 + jj) * k.D + kk + H] = g1[jj];
+  for (int q = 0; q < kPairRows / 2; ++q) {
+    float* lo = k.gneg + static_cast<size_t>(col0 + 2 * q) * k.D;
+    float* hi = lo + k.D;
+    unpack2(g0[q], lo[kk], hi[kk]);
+    unpack2(g1[q], lo[kk + H], hi[kk + H]);
   }
 }
 

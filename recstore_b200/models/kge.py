@@ -27,6 +27,7 @@ Checkpoints keep the reference layout (tensor_models.py:452-476, general_models.
 """
 from __future__ import annotations
 
+import contextlib
 import json
 import os
 from dataclasses import asdict, dataclass
@@ -148,6 +149,8 @@ class KGEModel:
         self._g_ids = (self.ids[:bs], torch.zeros(bs, dtype=torch.int64, device=dev), self.ids[bs:2 * bs], self.ids[2 * bs:])
         self._g_loss = torch.zeros((), **f)
         self._cap_stream: Optional[torch.cuda.Stream] = None
+        self._side: Optional[torch.cuda.Stream] = None        # second branch of a captured step
+        self._fork = False
 
     # ------------------------------------------------------------------ kernels
     def _stage(self, stage: int, corrupt_head: bool, want_scores: bool):
@@ -160,9 +163,25 @@ class KGEModel:
                   ptr(self.colsum), ptr(self.GA), ptr(self.GB), ptr(self.pos_score) if want_scores else None,
                   ptr(self.neg_score) if want_scores else None, stream_ptr())
 
+    @contextlib.contextmanager
+    def _beside(self):
+        """What is launched inside runs beside what follows, until :meth:`_join`.  Only in a captured step of one rank: a step is
+        some fifteen kernels of a few microseconds, and the relation table's halves, the accumulators' fill and one of the
+        two gradient GEMMs depend on nothing in between.  (Tables of several ranks share flag channels, and eager launches
+        would pay more for the events than they gain.)"""
+        if not self._fork:
+            yield
+            return
+        self._side.wait_stream(torch.cuda.current_stream())
+        with torch.cuda.stream(self._side):
+            yield
+
+    def _join(self):
+        if self._fork:
+            torch.cuda.current_stream().wait_stream(self._side)
+
     def _forward(self, corrupt_head: bool, want_scores: bool):
         st = self.ctx.status
-        self._sums.zero_()
         self._stage(0, corrupt_head, want_scores)
         if not self.pairwise:
             F_.gemm_bf16(self.A, self.Bn, self.S, mode=0, epi=F_.EPI_F32, status=st)
@@ -172,12 +191,15 @@ class KGEModel:
         bs = self.bs
         if h_ids is not self._g_ids[0]:
             self.ids[:bs].copy_(h_ids); self.ids[bs:2 * bs].copy_(t_ids); self.ids[2 * bs:].copy_(neg_ids)
+        with self._beside():
+            self._sums.zero_()
+            if self.rescal:
+                self._rel_keys.copy_((r_ids.view(-1, 1) * self.D + self._row_of_block).view(-1))
+                self.relation.lookup(self._rel_keys, out=self.rel_rows.view(self.bs * self.D, self.D))
+            else:
+                self.relation.lookup(r_ids.contiguous(), out=self.rel_rows)
         self.entity.lookup(self.ids, out=self.ent_rows)
-        if self.rescal:
-            self._rel_keys.copy_((r_ids.view(-1, 1) * self.D + self._row_of_block).view(-1))
-            self.relation.lookup(self._rel_keys, out=self.rel_rows.view(self.bs * self.D, self.D))
-        else:
-            self.relation.lookup(r_ids.contiguous(), out=self.rel_rows)
+        self._join()
         if self.transr:
             self._rel_keys.copy_((r_ids.view(-1, 1) * self.D + self._row_of_block).view(-1))
             self.proj.lookup(self._rel_keys, out=self.proj_rows)
@@ -246,8 +268,14 @@ class KGEModel:
                     self._cap_stream = torch.cuda.Stream()
                 self._cap_stream.wait_stream(cur)
                 cur = self._cap_stream
-            with torch.cuda.graph(g, stream=cur, capture_error_mode="relaxed"):
-                self._g_loss.copy_(self._step(*self._g_ids, corrupt_head))
+            if self._side is None:
+                self._side = torch.cuda.Stream()
+            self._fork = self.ctx.world == 1
+            try:
+                with torch.cuda.graph(g, stream=cur, capture_error_mode="relaxed"):
+                    self._g_loss.copy_(self._step(*self._g_ids, corrupt_head))
+            finally:
+                self._fork = False
             self._graphs[corrupt_head] = g
             return self._g_loss.clone()                       # the eager pass above already did this step's update
         self._graphs[corrupt_head].replay()
@@ -260,15 +288,19 @@ class KGEModel:
             return self._transr_step(corrupt_head)
         self._forward(corrupt_head, False)
         if not self.pairwise:
-            F_.gemm_bf16(self.W, self.Bn, self.GA, mode=2, epi=F_.EPI_F32, status=st)
+            with self._beside():
+                F_.gemm_bf16(self.W, self.Bn, self.GA, mode=2, epi=F_.EPI_F32, status=st)
             F_.gemm_bf16(self.W, self.A, self.GB, mode=1, epi=F_.EPI_F32, status=st)
+            self._join()
         self._stage(2, corrupt_head, False)
+        with self._beside():
+            if self.rescal:   # rowsum holds |dM|^2 of every positive: / D makes the table's mean over a row the mean over the matrix
+                self._rel_norm.copy_((self.rowsum / self.D).view(-1, 1).expand(self.bs, self.D).reshape(-1))
+                self.relation.update(self.rel_grad.view(self.bs * self.D, self.D), norms=self._rel_norm)
+            else:
+                self.relation.update(self.rel_grad)
         self.entity.update(self.ent_grad)
-        if self.rescal:   # rowsum holds |dM|^2 of every positive: / D makes the table's mean over a row the mean over the matrix
-            self._rel_norm.copy_((self.rowsum / self.D).view(-1, 1).expand(self.bs, self.D).reshape(-1))
-            self.relation.update(self.rel_grad.view(self.bs * self.D, self.D), norms=self._rel_norm)
-        else:
-            self.relation.update(self.rel_grad)
+        self._join()
         self.launches_per_step = (5 if self.pairwise else 7) + self.entity.launches + self.relation.launches
         return self.loss.sum()
 
