@@ -163,11 +163,11 @@ struct InterBwdArgs {
   int rows;                   // 0 = every row; 1 = only feature 0 (dx); 2 = only the embedding rows (pushed to their owners)
 };
 
-constexpr int kWarpsBwd = 6;  // 17 KB of shared memory per warp: two CTAs (12 warps) per SM
-constexpr int kOutLd = 72;    // staging row: 64 columns + 8 pad (144 B, 16-byte aligned, conflict-free)
+constexpr int kWarpsBwd = 4;  // 12 KB of shared memory per warp: four CTAs (16 warps) per SM
 constexpr int kDoutMax = kMaxD + kMaxF * (kMaxF - 1) / 2 + 16;
-// per-warp shared memory of the backward kernel (bytes): T tile, symmetric dZ, output staging, dOut row
-constexpr int kBwdWarpBytes = 32 * kLd * 2 + 32 * 40 * 2 + 32 * kOutLd * 2 + kDoutMax * 2;
+// per-warp shared memory of the backward kernel (bytes): T tile (results are staged in the columns already consumed),
+// symmetric dZ, dOut row
+constexpr int kBwdWarpBytes = 32 * kLd * 2 + 32 * 40 * 2 + kDoutMax * 2;
 
 __device__ __forceinline__ void stmatrix_x4(void* p, uint32_t r0, uint32_t r1, uint32_t r2, uint32_t r3) {
   const uint32_t a = static_cast<uint32_t>(__cvta_generic_to_shared(p));
@@ -180,10 +180,15 @@ __device__ __forceinline__ uint32_t pack2(float a, float b) {
 }
 
 // Persistent warps: every warp walks samples b = first, first + stride, ...  Everything that does not depend on
-// the sample (pair -> (i, j) table, destination pointers of the rows a lane stores) is set up once.
-__global__ void __launch_bounds__(kWarpsBwd * 32) interaction_bwd_kernel(const InterBwdArgs a) {
+// the sample (pair -> (i, j) table, destinations of the rows) is set up once per CTA, in shared memory.
+// Bound by instruction latency at few warps: 970 MB at 65,536 x 27 x 128 would take 146 us.  The results of a 64-column block
+// are staged over the columns of T that the block has just consumed, and the destination table lies in shared memory, which
+// makes room for 16 warps per SM (128 registers, no spills) instead of 12: 217 -> 208 us.  18 warps at 96 registers spill: 239 us.
+__global__ void __launch_bounds__(kWarpsBwd * 32, 4) interaction_bwd_kernel(const InterBwdArgs a) {
   extern __shared__ __align__(16) unsigned char smem_bwd[];
   __shared__ unsigned short s_ij[kMaxF * (kMaxF - 1) / 2];
+  __shared__ __nv_bfloat16* s_dst[kMaxF];   // destination of row i for sample 0 of this rank, or null
+  __shared__ float* s_nrm[kMaxF];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int F = a.F, D = a.D;
   const int npairs = F * (F - 1) / 2;
@@ -196,34 +201,31 @@ __global__ void __launch_bounds__(kWarpsBwd * 32) interaction_bwd_kernel(const I
   unsigned char* base = smem_bwd + warp * kBwdWarpBytes;
   __nv_bfloat16* t = reinterpret_cast<__nv_bfloat16*>(base);
   __nv_bfloat16* s = t + 32 * kLd;
-  __nv_bfloat16* o = s + 32 * 40;
-  __nv_bfloat16* sd = o + 32 * kOutLd;
+  __nv_bfloat16* sd = s + 32 * 40;
   for (int i = lane; i < 32 * 40 / 8; i += 32) reinterpret_cast<uint4*>(s)[i] = make_uint4(0, 0, 0, 0);
-  zero_tail_rows(t, F, D, lane);
+  if (threadIdx.x < kMaxF) {
+    const int i = threadIdx.x;
+    __nv_bfloat16* d = nullptr;
+    float* n = nullptr;
+    if (i == 0) {
+      if (a.rows != 2) d = a.dx;
+    } else if (i < F && a.rows != 1) {
+      const int f = i - 1;
+      d = reinterpret_cast<__nv_bfloat16*>(a.gdst[a.owner[f]]) + a.sample_base * a.grow_stride + a.gcol[f];
+      if (a.ndst) n = a.ndst[a.owner[f]] + a.sample_base * a.nstride + a.gcol[f] / D;
+    }
+    s_dst[i] = d;
+    s_nrm[i] = n;
+  }
   __syncthreads();
 
   const int g = lane >> 2, q = lane & 3;
   const int orow = lane >> 3, ochunk = lane & 7;  // store phase: 4 rows x 8 chunks of 16 B per instruction
-  // destination of the rows this lane stores (row i = it * 4 + orow), without the per-sample offset
-  __nv_bfloat16* dst_base[8];
-  float* nrm_base[8];
-#pragma unroll
-  for (int it = 0; it < 8; ++it) {
-    const int i = it * 4 + orow;
-    dst_base[it] = nullptr;
-    nrm_base[it] = nullptr;
-    if (i == 0) {
-      if (a.rows != 2) dst_base[it] = a.dx + ochunk * 8;
-    } else if (i < F && a.rows != 1) {
-      const int f = i - 1;
-      dst_base[it] = reinterpret_cast<__nv_bfloat16*>(a.gdst[a.owner[f]]) + a.sample_base * a.grow_stride + a.gcol[f] + ochunk * 8;
-      if (a.ndst) nrm_base[it] = a.ndst[a.owner[f]] + a.sample_base * a.nstride + a.gcol[f] / D;
-    }
-  }
   const int dvec = (a.dout_ld * 2) >> 4;  // uint4 per dOut row
 
   for (int b = blockIdx.x * kWarpsBwd + warp; b < a.B; b += gridDim.x * kWarpsBwd) {
     load_tile_async(t, a.T + static_cast<size_t>(b) * F * D, F, D, lane);
+    zero_tail_rows(t, F, D, lane);            // the previous sample's results were staged there
     const __nv_bfloat16* dout = a.dout + static_cast<size_t>(b) * a.dout_ld;
     for (int v = lane; v < dvec; v += 32) cp_async16(sd + v * 8, dout + v * 8);
     cp_async_wait_all();
@@ -287,12 +289,14 @@ __global__ void __launch_bounds__(kWarpsBwd * 32) interaction_bwd_kernel(const I
           }
         }
       }
-      // fragments -> staging tile: one stmatrix.x4 per (m-tile, pair of n-tiles)
+      // fragments -> staging, over the columns of T consumed above: one stmatrix.x4 per (m-tile, pair of n-tiles)
+      __syncwarp();
 #pragma unroll
       for (int mt = 0; mt < 2; ++mt)
 #pragma unroll
         for (int np = 0; np < 4; ++np) {
-          __nv_bfloat16* dstm = o + (mt * 16 + (lane & 7) + ((lane >> 3) & 1) * 8) * kOutLd + (np * 2 + (lane >> 4)) * 8;
+          if (n0 + np * 16 >= D) continue;
+          __nv_bfloat16* dstm = t + (mt * 16 + (lane & 7) + ((lane >> 3) & 1) * 8) * kLd + n0 + (np * 2 + (lane >> 4)) * 8;
           stmatrix_x4(dstm, pack2(acc[mt][np * 2][0], acc[mt][np * 2][1]), pack2(acc[mt][np * 2][2], acc[mt][np * 2][3]),
                       pack2(acc[mt][np * 2 + 1][0], acc[mt][np * 2 + 1][1]), pack2(acc[mt][np * 2 + 1][2], acc[mt][np * 2 + 1][3]));
         }
@@ -301,9 +305,10 @@ __global__ void __launch_bounds__(kWarpsBwd * 32) interaction_bwd_kernel(const I
       if (n0 + ochunk * 8 < D) {
 #pragma unroll
         for (int it = 0; it < 8; ++it) {
-          if (dst_base[it] == nullptr) continue;
           const int i = it * 4 + orow;
-          const uint4 v = *reinterpret_cast<const uint4*>(o + i * kOutLd + ochunk * 8);
+          __nv_bfloat16* const dst = s_dst[i];
+          if (dst == nullptr) continue;
+          const uint4 v = *reinterpret_cast<const uint4*>(t + i * kLd + n0 + ochunk * 8);
           const __nv_bfloat162* vp = reinterpret_cast<const __nv_bfloat162*>(&v);
           float sq = 0.f;
 #pragma unroll
@@ -313,7 +318,7 @@ __global__ void __launch_bounds__(kWarpsBwd * 32) interaction_bwd_kernel(const I
           }
           rownorm[it] += sq;
           const long long off = (i == 0) ? static_cast<long long>(b) * a.dx_ld : static_cast<long long>(b) * a.grow_stride;
-          *reinterpret_cast<uint4*>(dst_base[it] + off + n0) = v;
+          *reinterpret_cast<uint4*>(dst + off + n0 + ochunk * 8) = v;
         }
       }
       __syncwarp();
@@ -325,7 +330,8 @@ __global__ void __launch_bounds__(kWarpsBwd * 32) interaction_bwd_kernel(const I
         sq += __shfl_xor_sync(0xffffffffu, sq, 1);
         sq += __shfl_xor_sync(0xffffffffu, sq, 2);
         sq += __shfl_xor_sync(0xffffffffu, sq, 4);
-        if (ochunk == 0 && nrm_base[it] != nullptr) nrm_base[it][static_cast<long long>(b) * a.nstride] = sq;
+        float* const nrm = s_nrm[it * 4 + orow];
+        if (ochunk == 0 && nrm != nullptr) nrm[static_cast<long long>(b) * a.nstride] = sq;
       }
     }
   }
@@ -456,7 +462,7 @@ RS_API int rs_interaction_backward(const void* T, const void* dout, int B, int F
     attr_done = true;
   }
   int grid = (B + kWarpsBwd - 1) / kWarpsBwd;
-  if (grid > 148 * 4) grid = 148 * 4;   // persistent: warps loop over the samples
+  if (grid > 148 * 4) grid = 148 * 4;   // persistent: one resident wave, warps loop over the samples
   interaction_bwd_kernel<<<grid, kWarpsBwd * 32, smem, stream>>>(a);
   RS_LAUNCH_CHECK();
   return RS_OK;
