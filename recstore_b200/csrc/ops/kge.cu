@@ -26,8 +26,8 @@
 //                 GA = W . Neg (mode 2), GB = W^T . A (mode 1)
 //   kge_finish  : GA, GB -> gradients of x, r and of the negative entities
 // Pairwise family (TransE_l1, RotatE): sum |a - e'| is not a contraction, so three fp32 kernels walk
-// the (positive, negative) pairs of each chunk: kge_pair_forward (a warp per 4 x 8 pairs),
-// kge_pair_grad_pos (a thread per element of 8 positives, looping over the chunk's negatives) and
+// the (positive, negative) pairs of each chunk: kge_pair_forward (a warp per 4 x 4 pairs),
+// kge_pair_grad_pos (four threads per element of 8 positives, sharing the chunk's negatives) and
 // kge_pair_grad_neg (the transpose).  No atomics on the gradients: every output element has one owner.
 #include <cuda_bf16.h>
 #include "common/rs_common.h"
@@ -164,7 +164,7 @@ __device__ __forceinline__ float pair_dist(int model, float d0, float d1) {
 // ---- rows in 16-byte pieces (KgeArgs::vec) ---------------------------------------------------------------------------
 // A warp walks a row of a few hundred floats; loads of kRowBatch pieces per lane are issued before the first is used.  (One
 // element per lane and step, with stores between the loads, made the row kernels chains of a dozen memory latencies: prepare
-// 12.7 us and finish 17 us for 2,048 rows of 400.)
+// 12.7 us and finish 17 us for 2,048 rows of 400; now 5.7 and 5.9.)
 constexpr int kRowBatch = 4;
 __device__ __forceinline__ float4 add4(const float4& a, const float4& b, float s = 1.f) {
   return make_float4(a.x + s * b.x, a.y + s * b.y, a.z + s * b.z, a.w + s * b.w);
@@ -453,7 +453,7 @@ __global__ void __launch_bounds__(256) kge_prepare_kernel(const KgeArgs k) {
 // W row-major [bs, C*ns], zero outside the chunk diagonal.  A block takes 8 positives (one per warp) x 256 columns, a lane 8
 // neighbouring columns: row sums leave with one atomic per warp, column sums meet in shared memory over the 8 rows and leave
 // with one atomic per column, the loss with one per block.  (A thread per element with two global atomics each spent 37 us
-// on 524,288 atomics for 1,024 x 256 pairs; a block off the diagonal only writes zeros.)
+// on 524,288 atomics for 1,024 x 256 pairs, this form 6; a block off the diagonal only writes zeros.)
 constexpr int kLossCols = 256;
 __global__ void __launch_bounds__(256) kge_neg_loss_kernel(const KgeArgs k) {
   __shared__ float s_w[8][kLossCols];
@@ -675,7 +675,7 @@ __global__ void __launch_bounds__(256) kge_finish_kernel(const KgeArgs k) {
 // A warp scores 4 positives against 4 negatives of their chunk: every lane strides over the element pairs and keeps
 // 16 partial distances, which a transposing butterfly reduces so that lanes 2 p and 2 p + 1 end with pair p = (p / 4, p % 4).
 // Bound by latency and issue slots, operands come from L1 / L2: 16 sums leave room for twice the warps that 4 x 8 pairs did
-// (114 registers, 23 % of the warps resident, 53 us for 1,024 x 256 pairs of 200 complex elements).
+// (114 registers, 23 % of the warps resident, 53 us for 1,024 x 256 pairs of 200 complex elements; now 37 us).
 constexpr int kPairTileI = 4, kPairTileJ = 4;
 template <int MODEL>
 __global__ void __launch_bounds__(256, 3) kge_pair_forward_kernel(const KgeArgs k) {
@@ -788,8 +788,9 @@ __device__ __forceinline__ void pair_join(f32x2 (&g0)[kPairRows / 2], f32x2 (&g1
 
 // The two gradient kernels: a block owns 8 rows of one side x 32 element pairs; its 4 warps walk a quarter of the
 // other side's rows of the chunk each and add up at the end, so every gradient element still has one owner and no atomics.
-// Bound by issue slots (about a dozen instructions and one special function per element of a pair); one way of 128 threads
-// left three quarters of the warps out: 167 and 159 us for 1,024 x 256 pairs of 200 complex elements, 9 % resident.
+// Bound by the latency of the other side's rows; one way of 128 threads left three quarters of the warps out: 167 and 159 us
+// for 1,024 x 256 pairs of 200 complex elements, 9 % resident.  Now 48 and 45 us, of which the special-function unit accounts
+// for 12; fetching four rows at a time instead of two cost registers and was slower (75 and 67 us).
 
 // Block = 8 positives of one chunk; chains d loss / d a (negatives and the positive) to x and r.
 template <int MODEL>

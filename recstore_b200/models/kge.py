@@ -138,7 +138,9 @@ class KGEModel:
         self.GB = torch.empty(self.nneg, self.Dp, **f)
         self.pos_score = torch.empty(self.bs, **f)
         self.neg_score = torch.empty(self.bs, self.ns, **f)
-        self.ids = torch.empty(n_ids, dtype=torch.int64, device=dev)
+        # ids of a step in one buffer, so that one launch fills it: heads, tails, negatives, relations
+        self._id_buf = torch.zeros(n_ids + self.bs, dtype=torch.int64, device=dev)
+        self.ids = self._id_buf[:n_ids]
         self.step_no = 0
         self.heartbeat = None                # utils/liveness.Heartbeat: checked on the host before every step when set
         self.heartbeat_timeout_s = 2.0
@@ -146,7 +148,7 @@ class KGEModel:
         self._graphs: Dict[bool, torch.cuda.CUDAGraph] = {}
         # fixed id buffers of the captured step: the entity ids where the lookup reads them
         bs = self.bs
-        self._g_ids = (self.ids[:bs], torch.zeros(bs, dtype=torch.int64, device=dev), self.ids[bs:2 * bs], self.ids[2 * bs:])
+        self._g_ids = (self.ids[:bs], self._id_buf[n_ids:], self.ids[bs:2 * bs], self.ids[2 * bs:])
         self._g_loss = torch.zeros((), **f)
         self._cap_stream: Optional[torch.cuda.Stream] = None
         self._side: Optional[torch.cuda.Stream] = None        # second branch of a captured step
@@ -256,8 +258,7 @@ class KGEModel:
         self.step_no += 1
         if not self.cfg.use_cuda_graph:
             return self._step(h_ids, r_ids, t_ids, neg_ids, corrupt_head)
-        for dst, src in zip(self._g_ids, (h_ids, r_ids, t_ids, neg_ids)):
-            dst.copy_(src, non_blocking=True)
+        self._put_ids(h_ids, r_ids, t_ids, neg_ids)
         if corrupt_head not in self._graphs:
             self._g_loss.copy_(self._step(*self._g_ids, corrupt_head))   # eager once (this step's update): one-time set-up happens here
             torch.cuda.current_stream().synchronize()
@@ -281,6 +282,15 @@ class KGEModel:
         self._graphs[corrupt_head].replay()
         return self._g_loss.clone()
 
+    def _put_ids(self, h_ids, r_ids, t_ids, neg_ids) -> None:
+        src = (h_ids, t_ids, neg_ids, r_ids)
+        if all(x.dtype == torch.int64 and x.device == self.dev and x.dim() == 1 for x in src) and \
+                h_ids.numel() == t_ids.numel() == r_ids.numel() == self.bs and neg_ids.numel() == self.nneg:
+            torch.cat(src, out=self._id_buf)
+        else:                                # another type, place or a broadcast: one copy each
+            for dst, x in zip(self._g_ids, (h_ids, r_ids, t_ids, neg_ids)):
+                dst.copy_(x, non_blocking=True)
+
     def _step(self, h_ids, r_ids, t_ids, neg_ids, corrupt_head: bool) -> torch.Tensor:
         st = self.ctx.status
         self._fetch(h_ids, r_ids, t_ids, neg_ids)
@@ -294,6 +304,7 @@ class KGEModel:
             self._join()
         self._stage(2, corrupt_head, False)
         with self._beside():
+            loss = self.loss.sum()
             if self.rescal:   # rowsum holds |dM|^2 of every positive: / D makes the table's mean over a row the mean over the matrix
                 self._rel_norm.copy_((self.rowsum / self.D).view(-1, 1).expand(self.bs, self.D).reshape(-1))
                 self.relation.update(self.rel_grad.view(self.bs * self.D, self.D), norms=self._rel_norm)
@@ -302,7 +313,7 @@ class KGEModel:
         self.entity.update(self.ent_grad)
         self._join()
         self.launches_per_step = (5 if self.pairwise else 7) + self.entity.launches + self.relation.launches
-        return self.loss.sum()
+        return loss
 
     @torch.no_grad()
     def score_batch(self, h_ids, r_ids, t_ids, neg_ids, corrupt_head: bool) -> Tuple[torch.Tensor, torch.Tensor]:
