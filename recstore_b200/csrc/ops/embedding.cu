@@ -195,8 +195,10 @@ __global__ void __launch_bounds__(256) emb_fwd_sharded_kernel(const EmbFwdArgs a
 }
 
 // Bags a sub-warp of L lanes takes at once: as many as its lanes can describe while their ids stay near one id per lane of a
-// warp, one bag from 17 ids on, never more than `cap`.
+// warp, one bag from 17 ids on, never more than `cap`, except that four one-id bags are one batch of loads anyway (and fewer
+// CTAs leave a GEMM beside a small lookup more SMs).
 template <int L> __device__ __forceinline__ int bags_per_task(long long h, int cap) {
+  if (h <= 1 && cap < 4) cap = 4;
   int nb = h <= 1 ? L : (h >= 17 ? 1 : 1 << (31 - __clz(static_cast<int>(32 / h))));
   nb = nb < L ? nb : L;
   return nb < cap ? nb : cap;
@@ -211,7 +213,8 @@ template <int L> __device__ __forceinline__ int bags_per_task(long long h, int c
 // Bound by issue slots and rows in flight (skewed ids hit L2): at 128 floats half a warp per row, 32-byte loads and 16-byte
 // bf16 stores.  The form before it (a warp per 32 bags whatever they held, 16-byte loads by a warp per row, destination
 // worked out per row) took 180 us for 65,536 x 26 one-id bags at Zipf 1.2 and 342 us for 8,192 x 26 bags of 214 ids a
-// sample, there with one table's 256 warps still running long after the others had ended.
+// sample, there with one table's 256 warps still running long after the others had ended; this one 122 and 106 us (436 MB of
+// bf16 rows written in the first case: 66 us at 6.65 TB/s).
 template <int V, int L, int NC>
 __global__ void __launch_bounds__(256, 3) emb_pool_kernel(const EmbFwdArgs a, const int nb_cap) {
   constexpr int G = 32 / L;
@@ -465,7 +468,8 @@ __device__ __forceinline__ void bag_of(const EmbBwdArgs& a, long long i, int& t,
 // registers, one lane per row and warp adds to a shared-memory hash, and one global atomic per distinct row of the CTA
 // follows.  Without the first fold the float adds in shared memory, compare-and-swap loops, are serialised by the hot rows of
 // a skewed id stream (49 us for 1.70 M occurrences at Zipf 1.2); without the second the global atomics on the hottest row are
-// (33 us for 262,144 occurrences at Zipf 1.1), and its sum becomes a chain of thousands of fp32 roundings.
+// (33 us for 262,144 occurrences at Zipf 1.1), and its sum becomes a chain of thousands of fp32 roundings.  With both: 36 and
+// 13 us.
 struct StateFold {
   unsigned long long key[2 * kStateMax];
   float val[2 * kStateMax];
@@ -630,7 +634,7 @@ __global__ void __launch_bounds__(256) emb_state_kernel(const EmbBwdArgs a, cons
 // fewer of them meet on the hot rows, which the L2 takes one after another.
 // Bound by latency (sort, then gradients) and by those atomics: 16-byte bf16 loads by half a warp per 128-float row.  The
 // form before it (256 occurrences, a warp per row, state read and root inside the loop, 32 % of the warps resident) took
-// 278 us for 1.70 M occurrences x 128 at Zipf 1.2.
+// 278 us for 1.70 M occurrences x 128 at Zipf 1.2; this one 141 us (436 MB of gradients: 66 us), 231 us with groups of 256.
 template <int V, int L, int NC, bool BF16>
 __global__ void __launch_bounds__(kApplyThreads) emb_apply_kernel(const EmbBwdArgs a, const int gs) {
   constexpr int kPer = kApplyPer;
@@ -823,22 +827,6 @@ __global__ void rows_gather_kernel(const float* __restrict__ w, const long long*
   if (i >= n) return;
   const int lane = threadIdx.x & 31;
   const long long r = rows[i];
-  for (int v = lane; v < (D >> 2); v += 32) {
-    const float4 x = r >= 0 ? __ldg(reinterpret_cast<const float4*>(w + r * D) + v) : make_float4(0.f, 0.f, 0.f, 0.f);
-    *(reinterpret_cast<float4*>(out + i * D) + v) = x;
-  }
-}
-// Same gather with the row range checked: rows >= total_rows give zeros and set RS_DEV_OOB_ROW in the status word.
-__global__ void rows_gather_checked_kernel(const float* __restrict__ w, long long total_rows, const long long* __restrict__ rows,
-                                           long long n, int D, float* __restrict__ out, unsigned long long* status) {
-  const long long i = static_cast<long long>(blockIdx.x) * (blockDim.x >> 5) + (threadIdx.x >> 5);
-  if (i >= n) return;
-  const int lane = threadIdx.x & 31;
-  long long r = rows[i];
-  if (r >= total_rows) {
-    if (lane == 0 && status) atomicOr(status, (unsigned long long)RS_DEV_OOB_ROW);
-    r = -1;
-  }
   for (int v = lane; v < (D >> 2); v += 32) {
     const float4 x = r >= 0 ? __ldg(reinterpret_cast<const float4*>(w + r * D) + v) : make_float4(0.f, 0.f, 0.f, 0.f);
     *(reinterpret_cast<float4*>(out + i * D) + v) = x;
@@ -1044,8 +1032,12 @@ int emb_backward_impl(float* weight, float* state, long long total_rows, const l
   // once a batch fills them; below, the barriers of the sort cost more than the warps gain (3,072 rows of 400: 15.5 us).
   auto launch = [&](auto kern, int L) {
     const int threads = nnz >= 296ll * kApplyThreads ? kApplyThreads : 128;
+    // bf16 gradients come from the DLRM engine, which runs this pass beside the GEMMs of the bottom MLP: a GEMM CTA needs an SM
+    // for itself, so a small batch must not put a CTA on each (600 x 10 occurrences: 375 CTAs made the step 3 us longer
+    // than 24 did, although the pass itself is 4 us shorter).
+    const int least = grad_bf16 ? 128 : (threads / 32) * (32 / L);
     int gs = threads * kApplyPer;
-    while (gs > (threads / 32) * (32 / L) && nnz < 296ll * gs) gs >>= 1;
+    while (gs > least && nnz < 296ll * gs) gs >>= 1;
     kern<<<static_cast<unsigned>((nnz + gs - 1) / gs), threads, 0, stream>>>(a, gs);
   };
 #define RS_LAUNCH_APPLY(V, L, NC)                                 \
@@ -1069,15 +1061,6 @@ RS_API int rs_rows_gather(const float* weight, const long long* rows, long long 
   RS_LAUNCH_CHECK();
   return RS_OK;
 }
-RS_API int rs_rows_gather_checked(const float* weight, long long total_rows, const long long* rows, long long n, int D, float* out,
-                                  unsigned long long* status, cudaStream_t stream) {
-  RS_REQUIRE(weight && rows && out && D % 4 == 0 && total_rows >= 0, "rs_rows_gather_checked: bad argument");
-  if (n == 0) return RS_OK;
-  rows_gather_checked_kernel<<<static_cast<unsigned>((n + 7) / 8), 256, 0, stream>>>(weight, total_rows, rows, n, D, out, status);
-  RS_LAUNCH_CHECK();
-  return RS_OK;
-}
-
 RS_API int rs_rows_scatter(float* weight, const long long* rows, long long n, int D, const float* in,
                            cudaStream_t stream) {
   RS_REQUIRE(weight && rows && in && D % 4 == 0, "rs_rows_scatter: bad argument");

@@ -38,7 +38,6 @@ _lib.register_signatures({
     "rs_shard_gather_push_rows": (i32, [vp, i64, vp, vp, vp, vp, i32, i32, i32, i64, C.POINTER(HashTableView), vp, vp]),
     "rs_shard_gather_push_rows_tiered": (i32, [vp, vp, i64, i64, vp, vp, vp, vp, i32, i32, i32, i64, vp, vp]),
     "rs_tiered_apply": (i32, [vp, vp, vp, vp, i64, i64, vp, i64, i32, vp, vp, f32, f32, i32, vp]),
-    "rs_rows_gather_checked": (i32, [vp, i64, vp, i64, i32, vp, vp, vp]),
     "rs_shard_local": (i32, [vp, i64, vp, i64, i32, vp, vp, vp, vp, vp, C.POINTER(HashTableView), i32, i32, f32, vp, vp, vp]),
     "rs_shard_unbucket_rows": (i32, [vp, vp, i64, i32, vp, i32, vp]),
     "rs_shard_push_grads": (i32, [vp, vp, i64, i32, i32, i64, vp, vp, vp, vp]),
