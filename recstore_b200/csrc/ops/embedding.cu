@@ -1008,13 +1008,13 @@ int emb_backward_impl(float* weight, float* state, long long total_rows, const l
   // looked at in the kernel, they are device values).
   const bool wide = rs::row_wide(weight, D) && (reinterpret_cast<uintptr_t>(grad) & (grad_bf16 ? 15 : 31)) == 0;
   if (optimizer == 1) {
-    // As many occurrences per CTA as keep every SM busy with two CTAs, 1,024 at most.
+    // As many occurrences per CTA as keep every SM busy, 1,024 at most: the fewer atomics a hot row gets, the more exact its sum.
     if (gnorm) {
-      const int rounds = nnz >= 1024 * 296 ? 4 : nnz >= 512 * 296 ? 2 : 1;
+      const int rounds = nnz >= 1024 * 148 ? 4 : nnz >= 512 * 148 ? 2 : 1;
       emb_state_norm_kernel<<<static_cast<unsigned>((nnz + 256 * rounds - 1) / (256 * rounds)), 256, 0, stream>>>(a, rounds);
     } else {
       auto launch = [&](auto kern, int L) {
-        int opw = 32, rounds = nnz >= 1024 * 296 ? 4 : nnz >= 512 * 296 ? 2 : 1;
+        int opw = 32, rounds = nnz >= 1024 * 148 ? 4 : nnz >= 512 * 148 ? 2 : 1;
         while (opw > 32 / L && nnz < 8ll * opw * 296) opw >>= 1;
         kern<<<static_cast<unsigned>((nnz + 8 * opw * rounds - 1) / (8 * opw * rounds)), 256, 0, stream>>>(a, opw, rounds);
       };

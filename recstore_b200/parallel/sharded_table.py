@@ -7,7 +7,8 @@ windows (``csrc/comm/shard_exchange.cu``); every kernel publishes its own flag w
 done and the consumer waits inside its own prologue, so a lookup is five launches (clear + unique,
 bucket-and-push keys, owner-side gather-and-push rows, unbucket-and-expand) and an update four
 (segment sum, push, optimizer state, apply).  Nothing is staged through the host and no collective is
-called.  Duplicate ids are folded before they travel (``unique_keys`` + ``segment_sum``), which
+called.  With one rank and its rows in HBM nothing travels: a lookup is one launch and an update two
+(``csrc/kv/local_shard.cu``).  Duplicate ids are folded before they travel (``unique_keys`` + ``segment_sum``), which
 matters for Zipf / power-law id streams.
 
 Storage of a shard: a dense array indexed by ``id // world`` (ids are row numbers 0..N-1), or, with
